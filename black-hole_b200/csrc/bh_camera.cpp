@@ -12,6 +12,7 @@
 // device only has to apply the per-ray remainder (bh_integrate.cuh).
 // ---------------------------------------------------------------------------
 #include <cmath>
+#include <limits>
 #include "bh_trace_params.h"
 
 namespace {
@@ -94,6 +95,12 @@ void fill(CamFrame<T>& f, const TraceParams& t, float3 pos, float Mf, float af, 
     const T rCap = (T)t.rCap, dPhi = (T)t.dPhi;
     f.M = M; f.a = a; f.Q2 = Q * Q; f.a2 = a * a; f.a2Q2 = f.a2 + f.Q2;
     f.capR = rCap * T(1.002f) + T(1e-3f);
+    // Delta (r) >= 2e-5 + 1e-5 M^2 above rPlain: twice its larger floor (1e-5), with room
+    // for the rounding of r (r - 2M) + a^2 + Q^2
+    {
+        const T d = M * M - f.a2Q2 + T(2e-5f) + T(1e-5f) * M * M;
+        f.rPlain = d > T(0) ? fmaxT(f.capR, M + sqrtT(d)) : f.capR;
+    }
     f.rFloor = fmaxT((T)t.rPlus, rCap);
     f.rFloor105 = f.rFloor * T(1.05f);
     f.escR = T(120) * M;
@@ -101,7 +108,7 @@ void fill(CamFrame<T>& f, const TraceParams& t, float3 pos, float Mf, float af, 
     f.k8dPhi = T(8.0f) * dPhi;
     f.i22dPhi = T(1) / (T(2.2f) * dPhi);
     f.rPh15 = T(1.5f) * (T)t.rPhoton;
-    f.outer13 = (T)t.diskOuter * T(1.3f);
+    f.outer13 = t.diskOn ? (T)t.diskOuter * T(1.3f) : -std::numeric_limits<T>::infinity();
     f.dPhi = dPhi;
     f.hMin = dPhi * T(0.03f);
     f.uHor = T(1) / fmaxT(rCap, T(1e-6f));

@@ -71,6 +71,7 @@ struct CamFrame
     T uHor, uEscape, invNineM;   // 1/max(rCap, 1e-6), 1/(120 M), 1/(9 M)
     T uPh;                       // 1 / max(1.5 r_photon, 3 M)
     T diskTime;
+    T rPlain;                    // above it Delta stays clear of its floors (and of the capture test)
 };
 
 struct TraceParams
@@ -114,6 +115,7 @@ struct TraceParams
     const unsigned* nRaysDev;     // non-null: the ray count is read here at kernel start
     const unsigned* outIndex;     // BH_OUT_ANCHOR, non-null: list position k writes record outIndex[k]
 
+    float slabH;                  // half height of the disk's slab (the chords' vertical cull)
     CamFrame<float> cf;           // FP32 integration
     CamFrame<double> cd;          // FP64 integration
 };
