@@ -203,6 +203,8 @@ TraceParams frameParams(const RenderParams& P, int outMode, void* out)
     t.maxSteps = P.maxSteps;
     t.diskOn = P.diskEnabled ? 1 : 0;
     t.diskInner = P.diskInner; t.diskOuter = P.diskOuter; t.diskTime = P.diskTime;
+    t.cullIn = P.diskInner * (1.f - 1e-5f);
+    t.cullOut = P.diskOuter * (1.f + 1e-5f);
     t.slabH = 0.16f * P.diskOuter;
     t.emisK = P.diskEmisScale; t.absK = P.diskAbsScale;
     t.spotsOn = P.hotSpotsEnabled ? 1 : 0;

@@ -115,6 +115,7 @@ struct TraceParams
     const unsigned* nRaysDev;     // non-null: the ray count is read here at kernel start
     const unsigned* outIndex;     // BH_OUT_ANCHOR, non-null: list position k writes record outIndex[k]
 
+    float cullIn, cullOut;        // disk radii with room for rounding (the chords' radius cull)
     float slabH;                  // half height of the disk's slab (the chords' vertical cull)
     CamFrame<float> cf;           // FP32 integration
     CamFrame<double> cd;          // FP64 integration
