@@ -11,13 +11,23 @@
 // double and rounded to float (correctly rounded; the host libm's float acos
 // differs from that by one ulp on some inputs, a few ulps of rPhoton).
 //
-// The ISCO scan visits r = rStart, rStart + dr, ... as a running float sum --
-// a sequential recurrence whose rounding fixes the visited radii.  Thread 0
-// generates the exact sequence into shared memory 1024 values at a time; the
-// CTA evaluates the circular-orbit energies of a chunk in parallel and keeps,
-// per thread, the first minimum in visiting order; a final reduction picks
-// the smallest energy, ties to the earliest radius, which is what the
-// sequential strict "E < bestE" loop selects.
+// The ISCO scan visits r = rStart, rStart + dr, ... as a running float sum whose
+// rounding fixes the visited radii, and keeps the first of the lowest energies.
+// Neither the sum nor the whole scan has to be walked:
+//   * inside one binade every radius is a multiple of the binade's ulp, and after
+//     the first sum there (which may round a tie by the parity it comes with) the
+//     rounded increment is the same until the binade ends, so the visited
+//     radii are a handful of exact arithmetic sequences (Segment);
+//   * of a hole with a horizon the energy of the circular orbits falls from the
+//     photon orbit to the ISCO and rises from there on, so every kStride-th radius
+//     is evaluated first, and then all radii between those within kWindow of the
+//     lowest.  Near the minimum the energies of neighbouring visits differ by less
+//     than their rounding, so the window is evaluated exactly as the scan does it.
+//     A naked singularity, or a hole without a valid coarse radius, gets the whole
+//     scan.
+// Bound: instruction issue (the IEEE divisions and roots of ~2,600 energies a hole)
+// with one thread's set-up before it.  13,824 holes: 4.39 ms with the running sum
+// (a chain of 12,000 dependent sums a hole) and the whole scan, 0.19 ms so.
 // ---------------------------------------------------------------------------
 #include <cmath>
 #include <cuda_runtime.h>
@@ -25,8 +35,10 @@
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr int kChunk = 1024;
+constexpr int kThreads = 128;
+constexpr int kStride = 16;           // coarse pass of the scan
+constexpr float kWindow = 1e-3f;      // relative: coarse radii this close to the lowest energy mark the window
+constexpr int kMaxSegments = 64;
 constexpr float kExtremal = 0.995f;
 constexpr float kNakedCap = 2.25f;
 constexpr float kSingCut = 0.05f;
@@ -101,22 +113,81 @@ __device__ bool orbitEnergy(float r, float M, float a, float Q, float& E)
     return true;
 }
 
+// The visits first .. first + n - 1 of the scan: r = start + i step, exactly.
+struct Segment
+{
+    float start, step;
+    int first, n;
+};
+
+// The visiting sequence of `for (r = rStart; r <= rEnd; r += dr)` as exact
+// arithmetic sequences; returns the number of segments, the visits in *total.
+__device__ int scan_segments(float rStart, float rEnd, float dr, Segment* seg, int* total)
+{
+    int m = 0, k = 0;
+    float r = rStart;
+    while (r <= rEnd && m < kMaxSegments)
+    {
+        // ulp of r's binade and its upper end, in ulps 2^24 (normal numbers)
+        const int e = max((__float_as_int(r) >> 23) & 255, 1);
+        const double perUlp = __hiloint2double((1023 + 150 - e) << 20, 0);
+        const float r1 = fa(r, dr), step = fs(fa(r1, dr), r1);
+        constexpr int top = 1 << 24;
+        const bool same = max((__float_as_int(r1) >> 23) & 255, 1) == e;
+        // the visit at r itself; then the constant increments from r1 on, if r1 is in the binade
+        seg[m++] = Segment{r, 0.f, k, 1};
+        ++k;
+        r = r1;
+        if (!same || !(r1 <= rEnd) || m >= kMaxSegments) continue;
+        const int i1 = (int)((double)r1 * perUlp), inc = (int)fmin((double)step * perUlp, (double)top);
+        if (inc < 1) break;
+        const int lim = (int)fmin((double)rEnd * perUlp, (double)(top - 1));   // last multiple a visit may take
+        const int n = (lim - i1) / inc + 1;
+        seg[m++] = Segment{r1, step, k, n};
+        k += n;
+        r = fa(__fmaf_rn((float)(n - 1), step, r1), dr);
+    }
+    *total = k;
+    return m;
+}
+
+__device__ __forceinline__ float visit(const Segment* seg, int& at, int k)
+{
+    while (k >= seg[at].first + seg[at].n) ++at;
+    return __fmaf_rn((float)(k - seg[at].first), seg[at].step, seg[at].start);
+}
+
+// Lowest energy of the CTA and the earliest visit that has it (thread 0's values).
+__device__ void cta_lowest(float& E, int& k, float* sE, int* sK)
+{
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+    {
+        const float e2 = __shfl_down_sync(0xffffffffu, E, o);
+        const int k2 = __shfl_down_sync(0xffffffffu, k, o);
+        if (e2 < E || (e2 == E && k2 < k)) { E = e2; k = k2; }
+    }
+    if ((threadIdx.x & 31) == 0) { sE[threadIdx.x >> 5] = E; sK[threadIdx.x >> 5] = k; }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < kThreads / 32; ++w)
+            if (sE[w] < E || (sE[w] == E && sK[w] < k)) { E = sE[w]; k = sK[w]; }
+}
+
 __global__ void __launch_bounds__(kThreads)
 derive_kernel(BHDeriveRequest* __restrict__ req, BHDerived* __restrict__ out, int n)
 {
-    __shared__ float rs[kChunk];
-    __shared__ float redE[kThreads];
-    __shared__ int redK[kThreads];
-    __shared__ int sCount;
-    __shared__ float sNext;
+    __shared__ Segment seg[kMaxSegments];
+    __shared__ float sE[kThreads / 32], sLow;
+    __shared__ int sK[kThreads / 32], sTotal, sLo, sHi;
     __shared__ BHDerived sD;
-    __shared__ float sM, sA, sQ, sRp;
+    __shared__ float sM, sRp, sA, sQ;
     const int i = blockIdx.x;
     if (i >= n) return;
 
-    if (threadIdx.x == 0)
-    {
-        BHDeriveRequest R = req[i];
+    if (threadIdx.x == 0 || threadIdx.x == 32)
+    {   // both validate; one sets up the scan, the other derives the closed-form radii
+        const BHDeriveRequest R = req[i];
         float M = R.M, aStar = R.aStar, q = R.q;
         BHDerived d{0.f, 0.f, 1.f, 0.f, 1.5f, 1.f, 3.f, 0, 0};
         if (!(M > 0.f) || !isfinite(M)) { M = 0.5f; d.clamped = 1; }
@@ -142,82 +213,93 @@ derive_kernel(BHDeriveRequest* __restrict__ req, BHDerived* __restrict__ out, in
         }
         d.a = fm(aEff, M);
         d.Q = fm(qEff, M);
-        if (fs(fs(fm(M, M), fm(d.a, d.a)), fm(d.Q, d.Q)) < 0.f) { d.naked = 1; d.rPlus = 0.f; d.rMinus = 0.f; }
-        else { d.rPlus = outerHorizon(M, d.a, d.Q); d.rMinus = innerHorizon(M, d.a, d.Q); }
-        d.rErgo = d.naked ? 0.f : ergoRadius(M, d.Q);
-        if (spinning(R.model))
-        {
-            d.rPhoton = (R.model == BH_KERR_NEWMAN) ? photonOrbitKN(M, aEff, qEff) : photonOrbitKerr(M, aEff);
-            if (d.rPlus > 0.f) { if (d.rPhoton < fm(d.rPlus, 1.02f)) d.rPhoton = fm(d.rPlus, 1.02f); }
-            else if (d.rPhoton < fm(fm(kSingCut, M), 2.f)) d.rPhoton = fm(3.f, M);
+        d.naked = fs(fs(fm(M, M), fm(d.a, d.a)), fm(d.Q, d.Q)) < 0.f ? 1 : 0;
+        d.rPlus = d.naked ? 0.f : outerHorizon(M, d.a, d.Q);
+        if (threadIdx.x == 0)
+        {   // iscoRadius
+            const float rp = d.naked ? fm(kSingCut, M) : d.rPlus;
+            sRp = rp;
+            sM = M;
+            sLo = 0x7fffffff;
+            sHi = -1;
+            scan_segments(rp > 1e-6f ? fm(rp, 1.02f) : fm(0.5f, M), fm(12.f, M), fm(0.001f, M), seg, &sTotal);
         }
         else
         {
-            d.rPhoton = photonSphere(M, d.Q);
-            if (d.naked && !(d.rPhoton > 0.f)) d.rPhoton = fm(3.f, M);
+            d.rMinus = d.naked ? 0.f : innerHorizon(M, d.a, d.Q);
+            d.rErgo = d.naked ? 0.f : ergoRadius(M, d.Q);
+            if (spinning(R.model))
+            {
+                d.rPhoton = (R.model == BH_KERR_NEWMAN) ? photonOrbitKN(M, aEff, qEff) : photonOrbitKerr(M, aEff);
+                if (d.rPlus > 0.f) { if (d.rPhoton < fm(d.rPlus, 1.02f)) d.rPhoton = fm(d.rPlus, 1.02f); }
+                else if (d.rPhoton < fm(fm(kSingCut, M), 2.f)) d.rPhoton = fm(3.f, M);
+            }
+            else
+            {
+                d.rPhoton = photonSphere(M, d.Q);
+                if (d.naked && !(d.rPhoton > 0.f)) d.rPhoton = fm(3.f, M);
+            }
+            sD = d;
+            sA = aStar;
+            sQ = q;
         }
-        // ISCO scan set-up (iscoRadius)
-        const bool horizon = fs(fs(fm(M, M), fm(d.a, d.a)), fm(d.Q, d.Q)) >= 0.f;
-        const float rp = horizon ? outerHorizon(M, d.a, d.Q) : fm(kSingCut, M);
-        sRp = rp;
-        sNext = rp > 1e-6f ? fm(rp, 1.02f) : fm(0.5f, M);
-        sD = d;
-        sM = M; sA = aStar; sQ = q;
-        req[i].M = M; req[i].aStar = aStar; req[i].q = q;
     }
     __syncthreads();
     const float M = sM, a = sD.a, Q = sD.Q;
-    const float rEnd = fm(12.f, M), dr = fm(0.001f, M);
+    const int total = sTotal;
     float bestE = 1e30f;
     int bestK = 0x7fffffff;
-    int base = 0;
-    while (true)
+    int lo = 0, hi = total;               // visits to evaluate
+    if (!sD.naked)
     {
-        if (threadIdx.x == 0)
-        {   // the exact visiting sequence of `for (r = rStart; r <= rEnd; r += dr)`
-            float r = sNext;
-            int c = 0;
-            while (c < kChunk && r <= rEnd) { rs[c++] = r; r = fa(r, dr); }
-            sCount = c;
-            sNext = r;
-        }
-        __syncthreads();
-        const int c = sCount;
-        for (int k = threadIdx.x; k < c; k += kThreads)
+        int at = 0;
+        for (int k = (int)threadIdx.x * kStride; k < total; k += kThreads * kStride)
         {
             float E;
-            if (orbitEnergy(rs[k], M, a, Q, E) && E < bestE) { bestE = E; bestK = base + k; }
+            if (orbitEnergy(visit(seg, at, k), M, a, Q, E) && E < bestE) { bestE = E; bestK = k; }
         }
-        base += c;
+        cta_lowest(bestE, bestK, sE, sK);
+        if (threadIdx.x == 0) sLow = bestE;
         __syncthreads();
-        if (c < kChunk) break;
-    }
-    redE[threadIdx.x] = bestE;
-    redK[threadIdx.x] = bestK;
-    __syncthreads();
-    for (int s = kThreads / 2; s > 0; s >>= 1)
-    {
-        if (threadIdx.x < s)
+        const float low = sLow;
+        if (low < 1e30f)
         {
-            const float e2 = redE[threadIdx.x + s];
-            const int k2 = redK[threadIdx.x + s];
-            if (e2 < redE[threadIdx.x] || (e2 == redE[threadIdx.x] && k2 < redK[threadIdx.x]))
+            const float top = low + kWindow * fabsf(low);
+            at = 0;
+            for (int k = (int)threadIdx.x * kStride; k < total; k += kThreads * kStride)
             {
-                redE[threadIdx.x] = e2;
-                redK[threadIdx.x] = k2;
+                float E;
+                if (orbitEnergy(visit(seg, at, k), M, a, Q, E) && E <= top)
+                {
+                    atomicMin(&sLo, k);
+                    atomicMax(&sHi, k);
+                }
             }
+            __syncthreads();
+            lo = max(sLo - kStride + 1, 0);
+            hi = min(sHi + kStride, total);
         }
+        bestE = 1e30f;
+        bestK = 0x7fffffff;
         __syncthreads();
     }
+    {
+        int at = 0;
+        for (int k = lo + (int)threadIdx.x; k < hi; k += kThreads)
+        {
+            float E;
+            if (orbitEnergy(visit(seg, at, k), M, a, Q, E) && E < bestE) { bestE = E; bestK = k; }
+        }
+    }
+    cta_lowest(bestE, bestK, sE, sK);
     if (threadIdx.x == 0)
     {
         const float rp = sRp;
         float best;
-        if (redK[0] != 0x7fffffff)
-        {   // radius of the winning index: replay the same running sum
-            float r = rp > 1e-6f ? fm(rp, 1.02f) : fm(0.5f, M);
-            for (int k = 0; k < redK[0]; ++k) r = fa(r, dr);
-            best = r;
+        if (bestK != 0x7fffffff)
+        {
+            int at = 0;
+            best = visit(seg, at, bestK);
         }
         else
         {
@@ -227,6 +309,7 @@ derive_kernel(BHDeriveRequest* __restrict__ req, BHDerived* __restrict__ out, in
         BHDerived d = sD;
         d.rIsco = best > floorR ? best : floorR;
         out[i] = d;
+        req[i].M = sM; req[i].aStar = sA; req[i].q = sQ;
     }
 }
 
