@@ -49,6 +49,10 @@ constexpr float kPolarCap = 1.0f / 64.0f;
 // step's polynomial sine starts at 1/16; nearer the axis the try would mostly fail).
 constexpr float kPlainSin = 0.07f;
 
+// Per-ray statistics a ray object keeps: none, all of a probe record, or only the
+// disk hit (the ray sets the surrogate is trained on).
+enum { STATS_NONE = 0, STATS_FULL = 1, STATS_HIT = 2 };
+
 // A finished ray as it waits for shading: outcome flags, the radiance gathered
 // from the disk, and the six state values from which the escape direction is
 // rebuilt at shading time (so the finishing lane only stores, and the
@@ -240,7 +244,7 @@ BH_DEV SphInit<T> sph_init(const TraceParams& P, const CamFrame<T>& F, vec3<T> d
 // MIXED: FP32 state and steps; FP64 initial data, whole steps in FP64 where
 // the Binet solution turns (u' would change sign within the step), and FP64
 // location of the equatorial crossing.
-template <class R, bool STATS, bool MIXED = false>
+template <class R, int STATS, bool MIXED = false>
 struct SphRay
 {
     using Real = R;
@@ -264,7 +268,8 @@ struct SphRay
         step = 0;
         tFlight = R(0);
         prevPos = tof3(P.camPos);
-        if (STATS) { tally.samples = 0; tally.hitR = 0.f; tally.hitG = 0.f; I0 = 0.0; }
+        if (STATS) { tally.samples = 0; tally.hitR = 0.f; tally.hitG = 0.f; }
+        if (STATS == STATS_FULL) I0 = 0.0;
         bool radial, inward;
         if constexpr (MIXED)
         {
@@ -287,7 +292,7 @@ struct SphRay
             return RAY_DONE;
         }
         phi = R(0);
-        if (STATS) I0 = binet((R)P.M, (R)P.Q * (R)P.Q, u, du);
+        if (STATS == STATS_FULL) I0 = binet((R)P.M, (R)P.Q * (R)P.Q, u, du);
         return RAY_LIVE;
     }
 
@@ -346,7 +351,7 @@ struct SphRay
             sincos_fast(phi, sp, cp);
             f3 pos = v3((float)((F.e1[0] * cp + e2x * sp) * r), (float)((F.e1[1] * cp + e2y * sp) * r),
                         (float)((F.e1[2] * cp + e2z * sp) * r));
-            disk_segment<STATS>(P, E, Lz, prevPos, pos, (float)(F.diskTime - tFlight), accum, trans, tally);
+            disk_segment<STATS != STATS_NONE>(P, E, Lz, prevPos, pos, (float)(F.diskTime - tFlight), accum, trans, tally);
             prevPos = pos;
         }
         ++step;
@@ -388,7 +393,7 @@ struct SphRay
         q.acc[0] = accum.x; q.acc[1] = accum.y; q.acc[2] = accum.z;
         q.trans = trans;
         q.f[0] = ud; q.f[1] = dud; q.f[2] = phid; q.f[3] = e2x; q.f[4] = e2y; q.f[5] = e2z;
-        if (STATS)
+        if (STATS == STATS_FULL)
         {
             st->steps = step; st->samples = tally.samples; st->maxHviol = 0.f;
             st->hitR = tally.hitR; st->hitG = tally.hitG;
@@ -636,7 +641,7 @@ BH_DEV bool kerr_rk4_plain(const CamFrame<float>& F, const KerrConsts<float>& k,
 // between steps; what does is to carry an FP64 state from the step that enters
 // the cap |sin th| < kPolarCap to the step that leaves it, so that is what
 // MIXED does (polar_passage_fp64).
-template <class R, bool STATS, bool MIXED = false>
+template <class R, int STATS, bool MIXED = false>
 struct KerrRay
 {
     using Real = R;
@@ -711,7 +716,7 @@ struct KerrRay
         if (STATS)
         {
             tally.samples = 0; tally.hitR = 0.f; tally.hitG = 0.f;
-            Q0 = carterQ(th, pth, F.a, E, Lz);
+            if (STATS == STATS_FULL) Q0 = carterQ(th, pth, F.a, E, Lz);
         }
         return RAY_LIVE;
     }
@@ -742,7 +747,7 @@ struct KerrRay
                             !((r >= F.escR) & (d1.r > R(0))) & (s > kPlainSin);
             if (__all_sync(__activemask(), in))
             {
-                if (STATS) note_violation(F);
+                if (STATS == STATS_FULL) note_violation(F);
                 const R h = step_size(P, F);
                 const R rS = r, thS = th, drS = d1.r, dthS = d1.th;
                 if (kerr_rk4_plain(F, k, h, r, th, ph, pr, pth, d1))
@@ -772,7 +777,7 @@ struct KerrRay
         if (!finite_p(((r + pr) + (pth + d1.r)) + d1.pr))
         { horizon = true; return true; }
         if (r <= F.capR) { horizon = true; return true; }
-        if (STATS) note_violation(F);
+        if (STATS == STATS_FULL) note_violation(F);
         if (r >= F.escR && d1.r > R(0)) { escaped = useDeriv = true; return true; }
 
         const R h = step_size(P, F);
@@ -899,7 +904,7 @@ struct KerrRay
         }
         const f3 pos = cart(rs, y, ph);
         if (trans > 0.01f)
-            disk_segment<STATS>(P, (float)k.E, (float)k.Lz, prevPos, pos, (float)(F.diskTime - tFlight), accum,
+            disk_segment<STATS != STATS_NONE>(P, (float)k.E, (float)k.Lz, prevPos, pos, (float)(F.diskTime - tFlight), accum,
                                 trans, tally);
         prevPos = pos;
         prevCart = true;
@@ -944,7 +949,7 @@ struct KerrRay
             q.f[3] = dl[0]; q.f[4] = dl[1]; q.f[5] = dl[2];
         }
         else { q.f[3] = d1.r; q.f[4] = d1.th; q.f[5] = d1.ph; }
-        if (STATS)
+        if (STATS == STATS_FULL)
         {
             st->steps = step; st->samples = tally.samples; st->maxHviol = maxHviol;
             st->hitR = tally.hitR; st->hitG = tally.hitG;
@@ -977,7 +982,7 @@ struct KerrRay
 // step that decided to enter is taken here, so the call advances at least one
 // step.  Returns true when the ray terminated.  Out of line: the FP32 step
 // loop keeps its register budget.
-template <class R, bool STATS, bool MIXED>
+template <class R, int STATS, bool MIXED>
 __device__ __noinline__ bool KerrRay<R, STATS, MIXED>::polar_passage_fp64(const TraceParams& P)
 {
     if constexpr (MIXED && std::is_same<R, float>::value)
@@ -995,7 +1000,8 @@ __device__ __noinline__ bool KerrRay<R, STATS, MIXED>::polar_passage_fp64(const 
         if (!prevCart) { prevPos = cart((R)prevPos.x, prevPos.y, (R)prevPos.z); prevCart = true; }
         d.prevPos = prevPos; d.prevCart = true; d.accum = accum; d.trans = trans; d.maxHviol = maxHviol;
         d.step = step; d.horizon = horizon; d.escaped = escaped; d.useDeriv = useDeriv;
-        if (STATS) { d.tally = tally; d.Q0 = Q0; }
+        if (STATS) d.tally = tally;
+        if (STATS == STATS_FULL) d.Q0 = Q0;
         bool done = false;
         // bounded by the step budget: every iteration takes a step or terminates
         while (!(done = d.advance(P)))

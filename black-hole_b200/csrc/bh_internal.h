@@ -36,6 +36,12 @@ cudaError_t bh_launch_trace(const TraceParams& P, int precision, bool stats, int
 cudaError_t bh_launch_batch(bool kerr, const TraceParams* views, const unsigned* tileBase, int n,
                             unsigned totalTiles, unsigned* counter, int blocksPerSm, cudaStream_t stream);
 
+// ray sets (bh_trace.cu): sort the rays of the units for tracing, then trace the
+// units of one metric family and write their inputs' targets (bh_sg_train.h)
+struct RaySet;
+cudaError_t bh_sort_ray_set(const RaySet& S, cudaStream_t stream);
+cudaError_t bh_trace_ray_set(const RaySet& S, bool kerr, unsigned* counter, cudaStream_t stream);
+
 // resident CTAs per SM of the FP32 tracing kernel of a model's family
 cudaError_t bh_trace_max_blocks(int model, int* out);
 
@@ -47,6 +53,10 @@ cudaError_t bh_device_alloc(void** p, size_t bytes);
 // when not null, `vblur` the finished (vertically blurred) bloom of the same size
 cudaError_t bh_launch_post(uchar4* out, const float4* accum, float4* hblur, float4* vblur, int W, int H,
                            const PostConsts& pc, cudaStream_t stream);
+
+// bhValidateAndDerive (no naked singularities) without the numeric ISCO scan (bh_params.cpp)
+struct BHDerived;
+BHDerived bh_derive_closed_form(int model, float& M, float& aStar, float& q);
 
 // frame constants of a sanitised view for the given output (bh_api.cpp), and
 // the CTAs per SM the view's metric family is tuned for

@@ -110,7 +110,7 @@ float iscoRadius(float M, float a, float Q)
     return best > floorR ? best : floorR;
 }
 
-BHDerived deriveHole(int model, float& M, float& aStar, float& q, bool allowNaked)
+BHDerived deriveHole(int model, float& M, float& aStar, float& q, bool allowNaked, bool isco = true)
 {
     BHDerived d{0.f, 0.f, 1.f, 0.f, 1.5f, 1.f, 3.f, 0, 0};
     if (!(M > 0.f) || !std::isfinite(M)) { M = 0.5f; d.clamped = 1; }
@@ -154,7 +154,7 @@ BHDerived deriveHole(int model, float& M, float& aStar, float& q, bool allowNake
         d.rPhoton = photonSphere(M, d.Q);
         if (d.naked && !(d.rPhoton > 0.f)) d.rPhoton = 3.f * M;
     }
-    d.rIsco = iscoRadius(M, d.a, d.Q);
+    if (isco) d.rIsco = iscoRadius(M, d.a, d.Q);
     return d;
 }
 
@@ -174,6 +174,11 @@ inline void fixInt(int& v, int lo, int hi, int def, bool& fixed)
 }
 
 }  // namespace
+
+BHDerived bh_derive_closed_form(int model, float& M, float& aStar, float& q)
+{
+    return deriveHole(model, M, aStar, q, false, false);
+}
 
 extern "C" void bhValidateAndDerive(int model, float* M, float* aStar, float* q, int allowNaked,
                                     BHDerived* out)

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <random>
 #include <vector>
@@ -70,20 +71,28 @@ void orbitCamera(RenderParams& P, float az, float el, float d, float fovDeg)
     P.aspect = (float)P.width / (float)P.height;
 }
 
-// applyBlackHole (src/main.cpp:97-134): derive, disk inner edge at the ISCO.
-void applyHole(RenderParams& P, int model, float aStar, float q)
+// applyBlackHole (src/main.cpp:97-134): derive, disk inner edge at the ISCO (which the
+// device has scanned, bhDeriveBatch: the host's radius bit for bit).
+void applyHole(RenderParams& P, int model, float aStar, float q, float rIsco)
 {
     float M = 0.5f, a = aStar, qq = q;
-    BHDerived d;
-    bhValidateAndDerive(model, &M, &a, &qq, 0, &d);
+    const BHDerived d = bh_derive_closed_form(model, M, a, qq);
     P.model = model;
     P.M = M;
     P.aSpin = d.a; P.Qc = d.Q;
     P.rPlus = d.rPlus; P.rPhoton = d.rPhoton; P.rErgo = d.rErgo;
     P.allowNaked = 0;
-    P.diskInner = d.rIsco;
+    P.diskInner = rIsco;
     P.diskOuter = 8.f;
 }
+
+// The random view parameters of a ray set.
+struct ViewDraw
+{
+    int model;
+    float a, q, r, incl, az, fov;
+    int spots;
+};
 
 // normalised scene inputs of a sanitised orbit-camera frame
 void sceneInputs(const RenderParams& P, float& aN, float& qN, float& rN, float& iN)
@@ -124,6 +133,15 @@ struct BHSurrogate
     bool critValid = false;
     CritKey critKey;
     float crit[kCritBins];
+    // ray sets: views and units of one launch (two sets in turn: the host fills one while the GPU
+    // traces the other), their rays' tracing order
+    cudaStream_t aux = nullptr;       // the spherical family beside the Kerr family
+    unsigned char* setHost[2] = {nullptr, nullptr};
+    unsigned char* setDev[2] = {nullptr, nullptr};
+    unsigned short* setOrder[2] = {nullptr, nullptr};
+    cudaEvent_t setDone[2] = {nullptr, nullptr};
+    size_t setUnits = 0;
+    bool setPinned = false;
     // batch buffers of the training loop
     float* bIn = nullptr;
     float* bTgt = nullptr;
@@ -147,6 +165,45 @@ struct BHSurrogate
 
 namespace {
 
+void freeRaySets(BHSurrogate* s)
+{
+    for (int k = 0; k < 2; ++k)
+    {
+        if (s->setHost[k] && s->setPinned) cudaFreeHost(s->setHost[k]);
+        else std::free(s->setHost[k]);
+        if (s->setDev[k]) cudaFree(s->setDev[k]);
+        if (s->setOrder[k]) cudaFree(s->setOrder[k]);
+        if (s->setDone[k]) cudaEventDestroy(s->setDone[k]);
+        s->setHost[k] = nullptr; s->setDev[k] = nullptr; s->setOrder[k] = nullptr; s->setDone[k] = nullptr;
+    }
+    s->setUnits = 0;
+}
+
+// Room for `units` units (of at most as many views) in `sets` of the two buffers.  The
+// host side is pinned only where two take turns (a single copy gains nothing from it and
+// pinning costs some ms).
+cudaError_t ensureRaySets(BHSurrogate* s, size_t units, int sets)
+{
+    const size_t bytes = units * (sizeof(RayView) + sizeof(RayUnit));
+    if (s->setUnits >= units && (sets < 2 || s->setHost[1])) return cudaSuccess;
+    freeRaySets(s);
+    cudaError_t e = cudaSuccess;
+    if (!s->aux) e = cudaStreamCreateWithFlags(&s->aux, cudaStreamNonBlocking);
+    for (int k = 0; k < sets && e == cudaSuccess; ++k)
+    {
+        s->setPinned = sets > 1;
+        if (s->setPinned) e = cudaMallocHost(reinterpret_cast<void**>(&s->setHost[k]), bytes);
+        else if (!(s->setHost[k] = static_cast<unsigned char*>(std::malloc(bytes)))) e = cudaErrorMemoryAllocation;
+        if (e == cudaSuccess) e = bh_device_alloc(reinterpret_cast<void**>(&s->setDev[k]), bytes);
+        if (e == cudaSuccess)
+            e = bh_device_alloc(reinterpret_cast<void**>(&s->setOrder[k]), units * BH_UNIT_RAYS * sizeof(unsigned short));
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->setDone[k], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) { freeRaySets(s); return e; }
+    s->setUnits = units;
+    return cudaSuccess;
+}
+
 void freeAll(BHSurrogate* s)
 {
     SgState& S = s->S;
@@ -156,8 +213,10 @@ void freeAll(BHSurrogate* s)
                   s->cellPix, s->cellGate, s->sampleDir, s->samplePix, s->blockOrder};
     for (void* p : ps)
         if (p) cudaFree(p);
+    freeRaySets(s);
     if (s->evFork) cudaEventDestroy(s->evFork);
     if (s->evJoin) cudaEventDestroy(s->evJoin);
+    if (s->aux) cudaStreamDestroy(s->aux);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
 }
@@ -584,41 +643,104 @@ cudaError_t bhSurrogateGenerate(BHSurrogate* s, long long rays, int views, unsig
         if (e == cudaSuccess) e = bh_device_alloc(reinterpret_cast<void**>(&S.dsTgt), (size_t)rays * 8 * sizeof(float));
         if (e != cudaSuccess) return e;
     }
-    float3* dirs = nullptr;
-    BHProbe* rec = nullptr;
-    if (e == cudaSuccess) e = bh_device_alloc(reinterpret_cast<void**>(&dirs), (size_t)R * sizeof(float3));
-    if (e == cudaSuccess) e = bh_device_alloc(reinterpret_cast<void**>(&rec), (size_t)R * sizeof(BHProbe));
+    // the views' random parameters, in order; every hole's ISCO on the device
     std::mt19937 g(seed);
-    for (int v = 0; v < views && e == cudaSuccess; ++v)
+    std::vector<ViewDraw> draws(views);
+    std::vector<BHDeriveRequest> req(views);
+    std::vector<BHDerived> holes(views);
+    for (int v = 0; v < views; ++v)
     {
-        const int model = (int)(g() % 4u);
-        float a = 0.f, q = 0.f;
-        do { a = uni(g, -0.998f, 0.998f); q = uni(g, 0.f, 0.6f); } while (a * a + q * q > 0.98f);
-        if (model == BH_SCHWARZSCHILD || model == BH_REISSNER_NORDSTROM) a = 0.f;
-        if (model == BH_SCHWARZSCHILD || model == BH_KERR) q = 0.f;
-        const float r = uni(g, 6.f, 60.f), incl = uni(g, 2.f, 88.f), az = uni(g, 0.f, 2.f * kPi);
-        const float fov = uni(g, 30.f, 90.f);
-        RenderParams P;
-        P.width = 1920; P.height = 1080;
-        applyHole(P, model, a, q);
-        orbitCamera(P, az, (90.f - incl) * kPi / 180.f, r, fov);
-        P.diskEnabled = 1; P.hotSpotsEnabled = (g() & 1u) ? 1 : 0;
-        P.dPhi = 0.012f; P.maxSteps = 2000;
-        P.accumMode = 0; P.sampleIndex = 0;
-        bhSanitizeRenderParams(&P);
-        float aN, qN, rN, iN;
-        sceneInputs(P, aN, qN, rN, iN);
-        const TraceParams tp = bh_frame_params(P, BH_OUT_PROBE, nullptr);
-        float* in = S.dsIn + (size_t)v * R * 8;
-        float* tgt = S.dsTgt + (size_t)v * R * 8;
-        e = sg_make_rays(tp, aN, qN, rN, iN, seed * 0x9E3779B1u + (unsigned)v * 0x85EBCA77u, dirs, in, (int)R,
-                         s->stream);
-        if (e == cudaSuccess) e = bhProbeRays(rec, dirs, (int)R, P, BH_PREC_FP32, s->stream);
-        if (e == cudaSuccess) e = sg_make_targets(rec, tp, tgt, (int)R, s->stream);
+        ViewDraw& d = draws[v];
+        d.model = (int)(g() % 4u);
+        d.a = 0.f; d.q = 0.f;
+        do { d.a = uni(g, -0.998f, 0.998f); d.q = uni(g, 0.f, 0.6f); } while (d.a * d.a + d.q * d.q > 0.98f);
+        if (d.model == BH_SCHWARZSCHILD || d.model == BH_REISSNER_NORDSTROM) d.a = 0.f;
+        if (d.model == BH_SCHWARZSCHILD || d.model == BH_KERR) d.q = 0.f;
+        d.r = uni(g, 6.f, 60.f);
+        d.incl = uni(g, 2.f, 88.f);
+        d.az = uni(g, 0.f, 2.f * kPi);
+        d.fov = uni(g, 30.f, 90.f);
+        d.spots = (g() & 1u) ? 1 : 0;
+        req[v] = BHDeriveRequest{d.model, 0.5f, d.a, d.q, 0};
     }
+    const size_t perView = ((size_t)R + BH_UNIT_RAYS - 1) / BH_UNIT_RAYS, units = (size_t)views * perView;
+    const size_t chunk = std::min<size_t>(units, 2048);       // units of a launch
+    if (e == cudaSuccess) e = ensureRaySets(s, chunk, units > chunk ? 2 : 1);
+    BHDeriveRequest* dReq = nullptr;
+    BHDerived* dHoles = nullptr;
+    if (e == cudaSuccess) e = bh_device_alloc(reinterpret_cast<void**>(&dReq), req.size() * sizeof(BHDeriveRequest));
+    if (e == cudaSuccess) e = bh_device_alloc(reinterpret_cast<void**>(&dHoles), req.size() * sizeof(BHDerived));
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(dReq, req.data(), req.size() * sizeof(BHDeriveRequest), cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) e = bhDeriveBatch(dReq, dHoles, views, s->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(holes.data(), dHoles, holes.size() * sizeof(BHDerived), cudaMemcpyDeviceToHost, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
-    if (dirs) cudaFree(dirs);
-    if (rec) cudaFree(rec);
+    if (dReq) cudaFree(dReq);
+    if (dHoles) cudaFree(dHoles);
+
+    int turn = 0;
+    for (size_t u0 = 0; u0 < units && e == cudaSuccess; u0 += chunk, turn ^= 1)
+    {
+        const size_t u1 = std::min(units, u0 + chunk);
+        const int v0 = (int)(u0 / perView), v1 = (int)((u1 - 1) / perView);   // views of the chunk
+        if (u0 >= 2 * chunk) e = cudaEventSynchronize(s->setDone[turn]);
+        if (e != cudaSuccess) break;
+        RayView* rv = reinterpret_cast<RayView*>(s->setHost[turn]);
+        RayUnit* ru = reinterpret_cast<RayUnit*>(rv + (v1 - v0 + 1));
+        for (int v = v0; v <= v1; ++v)
+        {
+            const ViewDraw& d = draws[v];
+            RenderParams P;
+            P.width = 1920; P.height = 1080;
+            applyHole(P, d.model, d.a, d.q, holes[v].rIsco);
+            orbitCamera(P, d.az, (90.f - d.incl) * kPi / 180.f, d.r, d.fov);
+            P.diskEnabled = 1; P.hotSpotsEnabled = d.spots;
+            P.dPhi = 0.012f; P.maxSteps = 2000;
+            P.accumMode = 0; P.sampleIndex = 0;
+            bhSanitizeRenderParams(&P);
+            RayView& V = rv[v - v0];
+            V.tp = bh_frame_params(P, BH_OUT_PROBE, nullptr);
+            sceneInputs(P, V.scene[0], V.scene[1], V.scene[2], V.scene[3]);
+            V.seed = seed * 0x9E3779B1u + (unsigned)v * 0x85EBCA77u;
+            V.row = v;
+        }
+        RaySet set{};
+        size_t k = 0;
+        for (int family = 1; family >= 0; --family)
+        {
+            for (size_t u = u0; u < u1; ++u)
+            {
+                const int v = (int)(u / perView);
+                const bool kerr = draws[v].model == BH_KERR || draws[v].model == BH_KERR_NEWMAN;
+                if (kerr == (family == 1)) ru[k++] = RayUnit{v - v0, (unsigned)(u % perView) * BH_UNIT_RAYS};
+            }
+            if (family == 1) set.nKerr = (int)k;
+        }
+        set.nUnits = (int)k;
+        set.views = reinterpret_cast<const RayView*>(s->setDev[turn]);
+        set.units = reinterpret_cast<const RayUnit*>(set.views + (v1 - v0 + 1));
+        set.perView = (unsigned)R;
+        set.order = s->setOrder[turn];
+        set.in = S.dsIn;
+        set.tgt = S.dsTgt;
+        unsigned *cKerr = nullptr, *cSph = nullptr;
+        e = cudaMemcpyAsync(s->setDev[turn], s->setHost[turn],
+                            (size_t)(v1 - v0 + 1) * sizeof(RayView) + k * sizeof(RayUnit), cudaMemcpyHostToDevice,
+                            s->stream);
+        if (e == cudaSuccess) e = bh_sort_ray_set(set, s->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(s->evFork, s->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s->aux, s->evFork, 0);
+        if (e == cudaSuccess) e = bh_device_counter(&cKerr);
+        if (e == cudaSuccess) e = bh_device_counter(&cSph);
+        if (e == cudaSuccess) e = bh_trace_ray_set(set, true, cKerr, s->stream);
+        if (e == cudaSuccess) e = bh_trace_ray_set(set, false, cSph, s->aux);
+        if (e == cudaSuccess) e = cudaEventRecord(s->evJoin, s->aux);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s->stream, s->evJoin, 0);
+        if (e == cudaSuccess) e = cudaEventRecord(s->setDone[turn], s->stream);
+    }
+    const cudaError_t e2 = cudaStreamSynchronize(s->stream);
+    if (e == cudaSuccess) e = e2;
     if (e == cudaSuccess) S.dsN = rays;
     return e;
 }

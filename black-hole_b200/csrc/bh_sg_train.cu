@@ -216,57 +216,6 @@ __global__ void gather_kernel(const float4* __restrict__ dsIn, const float4* __r
     tgt[2 * k] = dsTgt[2 * idx]; tgt[2 * k + 1] = dsTgt[2 * idx + 1];
 }
 
-// ---- the RK4-traced ray set ----------------------------------------------------------
-__device__ __forceinline__ unsigned hash_u32(unsigned x)
-{
-    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
-    return x;
-}
-
-struct ViewInputs
-{
-    float aN, qN, rN, iN;
-};
-
-__global__ void rays_kernel(const __grid_constant__ TraceParams P, ViewInputs vi, unsigned seed, float3* __restrict__ dirs,
-                            float* __restrict__ in, int R)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= R) return;
-    const unsigned h1 = hash_u32(seed ^ hash_u32((unsigned)k * 2u + 1u));
-    const unsigned h2 = hash_u32(h1 + 0x9e3779b9u);
-    const float fx = (float)(h1 >> 8) * (1.f / 16777216.f), fy = (float)(h2 >> 8) * (1.f / 16777216.f);
-    const f3 d = camera_ray(P, fx, fy);
-    dirs[k] = make_float3(d.x, d.y, d.z);
-    float* x = in + (size_t)k * 8;
-    x[0] = d.x * P.camRight.x + d.y * P.camRight.y + d.z * P.camRight.z;
-    x[1] = d.x * P.camUp.x + d.y * P.camUp.y + d.z * P.camUp.z;
-    x[2] = d.x * P.camFwd.x + d.y * P.camFwd.y + d.z * P.camFwd.z;
-    x[3] = vi.aN; x[4] = vi.qN; x[5] = vi.rN; x[6] = vi.iN; x[7] = 0.f;
-}
-
-__global__ void targets_kernel(const BHProbe* __restrict__ rec, const __grid_constant__ TraceParams P,
-                               float* __restrict__ tgt, int R)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= R) return;
-    const BHProbe& o = rec[k];
-    const bool disk = (o.accum[0] + o.accum[1] + o.accum[2]) > 0.f || o.trans < 1.f;
-    const int cls = disk ? kClsDisk : (o.outcome == 1 ? kClsEscaped : kClsCaptured);
-    float* t = tgt + (size_t)k * 8;
-    t[0] = (float)cls;
-    const float ex = o.escDir[0], ey = o.escDir[1], ez = o.escDir[2];
-    const float inv = rsqrtf(fmaxf(ex * ex + ey * ey + ez * ez, 1e-30f));
-    t[1] = (ex * P.camRight.x + ey * P.camRight.y + ez * P.camRight.z) * inv;
-    t[2] = (ex * P.camUp.x + ey * P.camUp.y + ez * P.camUp.z) * inv;
-    t[3] = (ex * P.camFwd.x + ey * P.camFwd.y + ez * P.camFwd.z) * inv;
-    const bool hit = o.diskR > 0.f;
-    t[4] = hit ? o.diskR * 0.125f : 0.f;
-    t[5] = hit ? logf(fmaxf(o.diskG, 1e-6f)) : 0.f;
-    t[6] = hit ? 1.f : 0.f;
-    t[7] = 0.f;
-}
-
 inline unsigned blocksFor(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 }  // namespace
@@ -410,19 +359,6 @@ cudaError_t sg_adam(SgState& S, float lr, cudaStream_t s)
                                                        c1, c2);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? sg_pack_weights(S, s) : e;
-}
-
-cudaError_t sg_make_rays(const TraceParams& P, float aN, float qN, float rN, float iN, unsigned seed, float3* dirs,
-                         float* in, int R, cudaStream_t s)
-{
-    rays_kernel<<<blocksFor(R, 256), 256, 0, s>>>(P, ViewInputs{aN, qN, rN, iN}, seed, dirs, in, R);
-    return cudaGetLastError();
-}
-
-cudaError_t sg_make_targets(const void* rec, const TraceParams& P, float* tgt, int R, cudaStream_t s)
-{
-    targets_kernel<<<blocksFor(R, 256), 256, 0, s>>>(reinterpret_cast<const BHProbe*>(rec), P, tgt, R);
-    return cudaGetLastError();
 }
 
 cudaError_t sg_gather(const SgState& S, unsigned seed, float* in, float* tgt, int n, cudaStream_t s)

@@ -60,7 +60,4 @@ void sg_free_batch(SgState& S);
 cudaError_t sg_forward_train(SgState& S, const float* in, int n, cudaStream_t s);
 cudaError_t sg_gradients(SgState& S, const float* in, const float* tgt, int n, cudaStream_t s);
 cudaError_t sg_adam(SgState& S, float lr, cudaStream_t s);
-cudaError_t sg_make_rays(const TraceParams& P, float aN, float qN, float rN, float iN, unsigned seed, float3* dirs,
-                         float* in, int R, cudaStream_t s);
-cudaError_t sg_make_targets(const void* rec, const TraceParams& P, float* tgt, int R, cudaStream_t s);
 cudaError_t sg_gather(const SgState& S, unsigned seed, float* in, float* tgt, int n, cudaStream_t s);

@@ -368,6 +368,160 @@ batch_kernel(const TraceParams* __restrict__ views, const unsigned* __restrict__
 }
 static_assert(sizeof(TraceParams) % 8 == 0, "TraceParams is copied in 8-byte words");
 
+// ---------------------------------------------------------------------------
+// Ray sets: random rays through many views, for the surrogate's training
+// ---------------------------------------------------------------------------
+// One launch per metric family over all the units' 32-ray groups instead of a
+// launch a view: a view's 4096 rays are 128 warps, and lasted as long as its
+// longest ray (0.7 ms) on a mostly idle GPU.  The rays are random, so a unit's
+// rays are first sorted by distance from the screen centre (the hole) and angle:
+// a group is then a piece of an annulus whose rays take similar paths.  Group g
+// takes rank g / units of unit g % units, so the groups round the shadow, whose
+// rays are longest, of all views come first.  Records go straight to the target
+// rows; no sky is shaded.  Bound: issue slots, and the longest ray's chain of steps
+// at the end.  96 views of 4096 rays: 71.6 ms with a launch a view, 3.2 ms so.
+
+BH_DEV unsigned hash_u32(unsigned x)
+{
+    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
+    return x;
+}
+
+// screen position of ray k of a view, uniform over the screen
+BH_DEV void ray_screen(unsigned seed, unsigned k, float& fx, float& fy)
+{
+    const unsigned h1 = hash_u32(seed ^ hash_u32(k * 2u + 1u));
+    const unsigned h2 = hash_u32(h1 + 0x9e3779b9u);
+    fx = (float)(h1 >> 8) * (1.f / 16777216.f);
+    fy = (float)(h2 >> 8) * (1.f / 16777216.f);
+}
+
+constexpr int kSortBins = 1024;       // 64 annuli of equal area x 16 sectors
+
+__global__ void __launch_bounds__(256) sort_rays_kernel(const __grid_constant__ RaySet S)
+{
+    __shared__ unsigned bins[kSortBins];
+    __shared__ unsigned short key[BH_UNIT_RAYS];
+    __shared__ unsigned part[8];
+    const RayUnit u = S.units[blockIdx.x];
+    const RayView& V = S.views[u.view];
+    const TraceParams& P = V.tp;
+    const unsigned n = min(BH_UNIT_RAYS, S.perView - u.first);
+    unsigned short* order = S.order + (size_t)blockIdx.x * BH_UNIT_RAYS;
+    for (int b = threadIdx.x; b < kSortBins; b += 256) bins[b] = 0u;
+    __syncthreads();
+    const float aspect = P.aspect, scale = 64.f / (0.25f * (aspect * aspect + 1.f));
+    for (unsigned k = threadIdx.x; k < n; k += 256u)
+    {
+        float fx, fy;
+        ray_screen(V.seed, u.first + k, fx, fy);
+        const f3 d = camera_ray(P, fx, fy);
+        float* x = S.in + ((size_t)V.row * S.perView + u.first + k) * 8;
+        float4 a, b;
+        a.x = d.x * P.camRight.x + d.y * P.camRight.y + d.z * P.camRight.z;
+        a.y = d.x * P.camUp.x + d.y * P.camUp.y + d.z * P.camUp.z;
+        a.z = d.x * P.camFwd.x + d.y * P.camFwd.y + d.z * P.camFwd.z;
+        a.w = V.scene[0];
+        b = make_float4(V.scene[1], V.scene[2], V.scene[3], 0.f);
+        reinterpret_cast<float4*>(x)[0] = a;
+        reinterpret_cast<float4*>(x)[1] = b;
+        const float cx = (fx - 0.5f) * aspect, cy = fy - 0.5f;
+        const int annulus = min((int)((cx * cx + cy * cy) * scale), 63);
+        const int sector = (int)((atan2f(cy, cx) * 0.15915494f + 0.5f) * 16.f) & 15;
+        key[k] = (unsigned short)(annulus * 16 + sector);
+        atomicAdd(&bins[key[k]], 1u);
+    }
+    __syncthreads();
+    // exclusive prefix sums of the bins: 4 a thread
+    unsigned c[4], sum = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { c[j] = bins[threadIdx.x * 4 + j]; sum += c[j]; }
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    unsigned run = sum;
+#pragma unroll
+    for (unsigned o = 1; o < 32u; o <<= 1)
+    {
+        const unsigned v = __shfl_up_sync(0xffffffffu, run, o);
+        if (lane >= o) run += v;
+    }
+    if (lane == 31u) part[warp] = run;
+    __syncthreads();
+    unsigned at = run - sum;
+    for (unsigned w = 0; w < warp; ++w) at += part[w];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { bins[threadIdx.x * 4 + j] = at; at += c[j]; }
+    __syncthreads();
+    for (unsigned k = threadIdx.x; k < n; k += 256u) order[atomicAdd(&bins[key[k]], 1u)] = (unsigned short)k;
+}
+
+// A finished ray's target row: class, escape direction in the camera basis, disk-hit
+// radius / 8 and log redshift factor.
+template <class Ray>
+BH_DEV void write_target(const TraceParams& P, const Ray& ray, f3 dir, float* row)
+{
+    PackedRay<float> q;
+    ray.pack(P, 0u, q, nullptr);
+    const bool escaped = (q.key & kRayEscaped) != 0u;
+    const f3 e = escaped && (q.key & kRayUseState) ? Ray::escape_dir(P, q) : dir;
+    const bool disk = (q.acc[0] + q.acc[1] + q.acc[2]) > 0.f || q.trans < 1.f;
+    const float inv = rsqrtf(fmaxf(e.x * e.x + e.y * e.y + e.z * e.z, 1e-30f));
+    const bool hit = ray.tally.hitR > 0.f;
+    float4 a, b;
+    a.x = disk ? 2.f : (escaped ? 0.f : 1.f);
+    a.y = (e.x * P.camRight.x + e.y * P.camRight.y + e.z * P.camRight.z) * inv;
+    a.z = (e.x * P.camUp.x + e.y * P.camUp.y + e.z * P.camUp.z) * inv;
+    a.w = (e.x * P.camFwd.x + e.y * P.camFwd.y + e.z * P.camFwd.z) * inv;
+    b.x = hit ? ray.tally.hitR * 0.125f : 0.f;
+    b.y = hit ? logf(fmaxf(ray.tally.hitG, 1e-6f)) : 0.f;
+    b.z = hit ? 1.f : 0.f;
+    b.w = 0.f;
+    reinterpret_cast<float4*>(row)[0] = a;
+    reinterpret_cast<float4*>(row)[1] = b;
+}
+
+template <class Ray>
+__global__ void __launch_bounds__(BH_TRACE_BLOCK, 5)
+ray_set_kernel(const __grid_constant__ RaySet S, int first, int nUnits, unsigned groups, unsigned* counter)
+{
+    __shared__ TraceParams sp[BH_TRACE_BLOCK / 32];
+    const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    TraceParams& P = sp[warp];
+    int cur = -1;
+    while (true)
+    {
+        unsigned g = 0;
+        if (lane == 0) g = atomicAdd(counter, 1u);
+        g = __shfl_sync(0xffffffffu, g, 0);
+        if (g >= groups) break;
+        const unsigned rank = g / (unsigned)nUnits;
+        const int ui = first + (int)(g - rank * (unsigned)nUnits);
+        const RayUnit u = S.units[ui];
+        const RayView& V = S.views[u.view];
+        if (u.view != cur)
+        {
+            const long long* src = reinterpret_cast<const long long*>(&V.tp);
+            long long* dst = reinterpret_cast<long long*>(&P);
+            for (int i = (int)lane; i < (int)(sizeof(TraceParams) / 8); i += 32) dst[i] = __ldg(src + i);
+            __syncwarp();
+            cur = u.view;
+        }
+        const unsigned at = rank * 32u + lane, n = min(BH_UNIT_RAYS, S.perView - u.first);
+        if (at < n)
+        {
+            const unsigned k = u.first + S.order[(size_t)ui * BH_UNIT_RAYS + at];
+            float fx, fy;
+            ray_screen(V.seed, k, fx, fy);
+            const f3 dir = camera_ray(P, fx, fy);
+            Ray ray;
+            bool live = ray.init(P, dir) == RAY_LIVE;
+            while (live)
+                if (ray.advance(P)) live = false;
+            write_target(P, ray, dir, S.tgt + ((size_t)V.row * S.perView + k) * 8);
+        }
+        __syncwarp();
+    }
+}
+
 template <class Ray, bool STATS>
 cudaError_t launch_one(const TraceParams& P, int blocksPerSm, cudaStream_t stream)
 {
@@ -443,6 +597,29 @@ cudaError_t bh_launch_batch(bool kerr, const TraceParams* views, const unsigned*
     const long long need = ((long long)totalTiles * 32 + block - 1) / block;
     if (grid > need) grid = need;
     k<<<(unsigned)grid, block, 0, stream>>>(views, tileBase, n, totalTiles, counter);
+    return cudaGetLastError();
+}
+
+cudaError_t bh_sort_ray_set(const RaySet& S, cudaStream_t stream)
+{
+    if (S.nUnits <= 0) return cudaSuccess;
+    sort_rays_kernel<<<S.nUnits, 256, 0, stream>>>(S);
+    return cudaGetLastError();
+}
+
+cudaError_t bh_trace_ray_set(const RaySet& S, bool kerr, unsigned* counter, cudaStream_t stream)
+{
+    const int first = kerr ? 0 : S.nKerr, nUnits = kerr ? S.nKerr : S.nUnits - S.nKerr;
+    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned), stream);
+    if (e != cudaSuccess || nUnits <= 0) return e;
+    const unsigned ranks = (min(BH_UNIT_RAYS, S.perView) + 31u) / 32u, groups = ranks * (unsigned)nUnits;
+    auto k = kerr ? ray_set_kernel<KerrRay<float, STATS_HIT>> : ray_set_kernel<SphRay<float, STATS_HIT>>;
+    int dev = 0, sms = 0, occ = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, BH_TRACE_BLOCK, 0)) != cudaSuccess) return e;
+    const unsigned need = (groups + BH_TRACE_BLOCK / 32u - 1u) / (BH_TRACE_BLOCK / 32u);
+    k<<<min(need, (unsigned)(max(occ, 1) * sms)), BH_TRACE_BLOCK, 0, stream>>>(S, first, nUnits, groups, counter);
     return cudaGetLastError();
 }
 

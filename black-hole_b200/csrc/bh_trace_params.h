@@ -120,3 +120,29 @@ struct TraceParams
     CamFrame<float> cf;           // FP32 integration
     CamFrame<double> cd;          // FP64 integration
 };
+
+// A set of random rays through several views (the rays the surrogate is trained
+// on).  The rays of a view are cut into units of BH_UNIT_RAYS; a unit's rays are
+// traced in an order of their own (`order`) and written at their own rows.
+constexpr unsigned BH_UNIT_RAYS = 4096u;
+struct RayView
+{
+    TraceParams tp;
+    float scene[4];               // normalised a*, q, log r, inclination
+    unsigned seed;
+    int row;                      // the view's number: its rays fill rows row * perView ...
+};
+struct RayUnit
+{
+    int view;                     // index into views
+    unsigned first;               // first ray of the unit within its view
+};
+struct RaySet
+{
+    const RayView* views;
+    const RayUnit* units;         // Kerr-family units first
+    int nKerr, nUnits;
+    unsigned perView;             // rays of a view
+    unsigned short* order;        // per unit: BH_UNIT_RAYS ray numbers, in tracing order
+    float *in, *tgt;              // rows of 8 floats
+};
