@@ -275,14 +275,15 @@ trace_kernel(const __grid_constant__ TraceParams P)
 // ---------------------------------------------------------------------------
 // Batched views: one persistent launch over the tiles of many views
 // ---------------------------------------------------------------------------
-// One tile (32 rays) of one view, traced by a whole warp: tile-synchronous, the
-// warp shades its 32 results together once every lane is done.
+// One tile (32 rays, or the part of one that `width` lanes take) of one view, traced by
+// a whole warp: tile-synchronous, the warp shades its results together once every
+// lane is done.
 template <class Ray>
-BH_DEV void trace_tile(const TraceParams& P, unsigned tile, unsigned lane, unsigned nRays)
+BH_DEV void trace_tile(const TraceParams& P, unsigned tile, unsigned lane, unsigned nRays, unsigned width)
 {
-    const unsigned rid = tile * 32u + lane;
+    const unsigned rid = tile * width + lane;
     int px = 0, py = 0;
-    const bool inFrame = rid < nRays && ray_pixel(P, rid, px, py);
+    const bool inFrame = lane < width && rid < nRays && ray_pixel(P, rid, px, py);
     Ray ray;
     bool live = false, fin = false;
     unsigned key = 0;
@@ -305,8 +306,9 @@ BH_DEV void trace_tile(const TraceParams& P, unsigned tile, unsigned lane, unsig
 }
 
 // One frame (or one pixel list), tile-synchronous: each warp claims 32 ray
-// ids -- one 8x4 tile, or 32 consecutive list entries -- at a time (the
-// counter counts tiles) and traces them to the last ray.  This is the FP32
+// ids -- one 8x4 tile, or 32 consecutive list entries; fewer where there are few
+// (rays_per_warp) -- at a time (the counter counts tiles) and traces them to the
+// last ray.  This is the FP32
 // render path under the default work distribution (a warp refills only when
 // all 32 lanes are idle); it skips trace_kernel's per-step ballots and result
 // ring.  Plain frames and the surrogate's RK4 pixel lists share this kernel,
@@ -317,14 +319,14 @@ tile_kernel(const __grid_constant__ TraceParams P)
 {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned nRays = P.nRaysDev ? min(*P.nRaysDev, P.nRays) : P.nRays;
-    const unsigned nTiles = (nRays + 31u) / 32u;
+    const unsigned width = (unsigned)P.raysPerWarp, nTiles = (nRays + width - 1u) / width;
     while (true)
     {
         unsigned t = 0;
         if (lane == 0) t = atomicAdd(P.counter, 1u);
         t = __shfl_sync(0xffffffffu, t, 0);
         if (t >= nTiles) break;
-        trace_tile<Ray>(P, t, lane, nRays);
+        trace_tile<Ray>(P, t, lane, nRays, width);
         __syncwarp();
     }
 }
@@ -362,7 +364,7 @@ batch_kernel(const TraceParams* __restrict__ views, const unsigned* __restrict__
             __syncwarp();
             cur = lo;
         }
-        trace_tile<Ray>(sp[warp], g - __ldg(tileBase + lo), lane, sp[warp].nRays);
+        trace_tile<Ray>(sp[warp], g - __ldg(tileBase + lo), lane, sp[warp].nRays, 32u);
         __syncwarp();
     }
 }
@@ -522,13 +524,36 @@ ray_set_kernel(const __grid_constant__ RaySet S, int first, int nUnits, unsigned
     }
 }
 
-template <class Ray, bool STATS>
-cudaError_t launch_one(const TraceParams& P, int blocksPerSm, cudaStream_t stream)
+// Rays a warp of the tile kernel takes at a time.  A small frame lasts as long as the
+// warp of its longest rays, and a warp's steps cost the union of its lanes' paths (disk
+// samples above all, which come at different steps); while the GPU has warps to
+// spare, fewer rays a warp shorten that.  The largest power of two that makes at most
+// 8192 groups (14 a scheduler): 128 x 72 Kerr-Newman 1.19 ms at 32 rays a warp, 1.05 /
+// 1.04 / 1.03 / 0.93 / 0.98 at 16 / 8 / 4 / 2 / 1 (2 taken); 320 x 180 1.92, 1.78 / 1.74 / 1.90 /
+// 2.09 / 3.75 (8 taken); 480 x 270 1.73, 1.64 / 1.76 / 2.32 (16 taken); 640 x 360 1.89, 1.88 /
+// 2.30 (32 taken); Reissner-Nordstroem 128 x 72 0.81 -> 0.47, 320 x 180 0.70 -> 0.59.
+// (A list whose length only the device knows is traced 32 at a time.)
+int rays_per_warp(const TraceParams& P)
 {
+    int width = 32;
+    if (!P.nRaysDev)
+        while (width > 1 && ((unsigned long long)P.nRays * 2u) / (unsigned)width <= 8192u) width >>= 1;
+    return width;
+}
+
+template <class Ray, bool STATS>
+cudaError_t launch_one(const TraceParams& P0, int blocksPerSm, cudaStream_t stream)
+{
+    TraceParams P = P0;
+    P.raysPerWarp = 32;
     auto k = trace_kernel<Ray, STATS>;
     if constexpr (!STATS && sizeof(typename Ray::Real) == 4)
     {   // whole frames under the default work distribution: tile-synchronous
-        if (P.refillMin >= 32 && !P.dirs) k = tile_kernel<Ray>;
+        if (P.refillMin >= 32 && !P.dirs)
+        {
+            k = tile_kernel<Ray>;
+            P.raysPerWarp = rays_per_warp(P);
+        }
     }
     int dev = 0, sms = 0, occ = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -540,7 +565,7 @@ cudaError_t launch_one(const TraceParams& P, int blocksPerSm, cudaStream_t strea
     if (e != cudaSuccess) return e;
     if (occ < 1) occ = 1;
     int per = (blocksPerSm > 0 && blocksPerSm < occ) ? blocksPerSm : occ;
-    long long need = ((long long)P.nRays + block - 1) / block;
+    long long need = ((long long)P.nRays * (32 / P.raysPerWarp) + block - 1) / block;
     long long grid = (long long)per * sms;
     if (grid > need) grid = need;
     if (grid < 1) grid = 1;

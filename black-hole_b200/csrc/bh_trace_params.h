@@ -110,6 +110,7 @@ struct TraceParams
     // work distribution
     unsigned* counter;            // ray counter, zeroed before the launch
     int refillMin;                // refill a warp when at least this many lanes are free
+    int raysPerWarp;              // rays a warp of the tile kernel takes at a time (set at the launch)
     const unsigned* tileOrder;    // non-null: k-th claimed tile -> tile index (trace order)
     const unsigned* pixList;      // non-null: ray k traces pixel pixList[k] (y * W + x)
     const unsigned* nRaysDev;     // non-null: the ray count is read here at kernel start
