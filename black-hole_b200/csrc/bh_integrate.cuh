@@ -249,6 +249,7 @@ struct SphRay
 {
     using Real = R;
     static constexpr bool kKerrFamily = false;
+    static constexpr bool kParks = false;
     R u, du, phi, tFlight, invB;
     R e2x, e2y, e2z;                  // in-plane unit vector normal to e1 (e1 is the camera's)
     R ud, dud, phid;                  // state of the last chord direction (deferred)
@@ -646,6 +647,7 @@ struct KerrRay
 {
     using Real = R;
     static constexpr bool kKerrFamily = true;
+    static constexpr bool kParks = MIXED;
     R r, th, ph, pr, pth;   // Boyer-Lindquist state
     R s, c;                 // sin/cos of th
     KerrConsts<R> k;        // E, Lz and their products
@@ -657,6 +659,7 @@ struct KerrRay
     int step;
     bool horizon, escaped, useDeriv;
     bool prevCart;          // prevPos holds (x, y, z); else (r sin th, y, ph) of the last point (FP32 rays)
+    bool parked;            // MIXED: the next step enters the polar cap (polar_passage_fp64 goes on from here)
     DiskTally tally;
     double Q0;
 
@@ -713,6 +716,7 @@ struct KerrRay
         maxHviol = 0.f;
         step = 0;
         horizon = escaped = useDeriv = false;
+        parked = false;
         if (STATS)
         {
             tally.samples = 0; tally.hitR = 0.f; tally.hitG = 0.f;
@@ -737,7 +741,7 @@ struct KerrRay
     BH_DEV bool advance(const TraceParams& P)
     {
         const CamFrame<R>& F = frame_of<R>(P);
-        if constexpr (std::is_same<R, float>::value && !MIXED)
+        if constexpr (std::is_same<R, float>::value)
         {   // the common step: nothing ends the ray here, no polar cap, no last step of the
             // budget (one test), and stage points that need no guard.  The whole warp takes it
             // or none does: lanes in both forms would run one after the other (a 640 x 360 frame,
@@ -784,7 +788,7 @@ struct KerrRay
         const R rS = r, thS = th, drS = d1.r, dthS = d1.th;    // step start (crossing search)
         if constexpr (MIXED)
         {
-            if (abs_p(s) < R(kPolarCap)) return polar_passage_fp64(P);
+            if (abs_p(s) < R(kPolarCap)) { parked = true; return false; }
         }
 
         KerrDeriv<R> d4;
@@ -979,8 +983,8 @@ struct KerrRay
 // termination tests and disk chords, E and Lz as the FP32 ray holds them) with
 // its state carried in FP64 from step to step, until it leaves the cap
 // |sin th| < kPolarCap or terminates; then the state is rounded back once.  The
-// step that decided to enter is taken here, so the call advances at least one
-// step.  Returns true when the ray terminated.  Out of line: the FP32 step
+// step that decided to enter (advance returned with `parked` set) is taken here, so
+// the call advances at least one step.  Returns true when the ray terminated.  Out of line: the FP32 step
 // loop keeps its register budget.
 template <class R, int STATS, bool MIXED>
 __device__ __noinline__ bool KerrRay<R, STATS, MIXED>::polar_passage_fp64(const TraceParams& P)
@@ -1011,8 +1015,8 @@ __device__ __noinline__ bool KerrRay<R, STATS, MIXED>::polar_passage_fp64(const 
         prevPos = d.prevPos; prevCart = true; accum = d.accum; trans = d.trans; maxHviol = d.maxHviol;
         step = d.step; horizon = d.horizon; escaped = d.escaped; useDeriv = d.useDeriv;
         if (STATS) tally = d.tally;
-        if (done && escaped && useDeriv && step >= P.maxSteps)
-        {   // budget exhausted inside the passage: the last stage's derivative
+        if (step >= P.maxSteps)
+        {   // budget spent in the passage, which the ray may have left: the last stage's derivative
             const double* dd = KerrRay<double, STATS, false>::last_deriv();
             R* dl = last_deriv();
             dl[0] = (R)dd[0]; dl[1] = (R)dd[1]; dl[2] = (R)dd[2];

@@ -164,6 +164,19 @@ __host__ __device__ constexpr int min_blocks()
     return Ray::kKerrFamily ? 5 : BH_TRACE_MIN_BLOCKS;
 }
 
+// The FP64 passage of a ray that waits for one; true when the ray has terminated.
+template <class Ray>
+BH_DEV bool pass_cap(const TraceParams& P, Ray& ray)
+{
+    if constexpr (Ray::kParks)
+    {
+        if (!ray.parked) return false;
+        ray.parked = false;
+        return ray.polar_passage_fp64(P);
+    }
+    return false;
+}
+
 template <class Ray, bool STATS>
 __global__ void __launch_bounds__(block_of<Ray, STATS>(), min_blocks<Ray, STATS>())
 trace_kernel(const __grid_constant__ TraceParams P)
@@ -236,7 +249,7 @@ trace_kernel(const __grid_constant__ TraceParams P)
         // two steps per scheduling round: halves the ballot / refill bookkeeping
 #pragma unroll 1
         for (int k = 0; k < 2; ++k)
-            if (live && ray.advance(P)) { live = false; fin = true; }
+            if (live && (ray.advance(P) || pass_cap(P, ray))) { live = false; fin = true; }
 
         const unsigned finMask = __ballot_sync(FULL, fin);
         if (finMask)
@@ -294,9 +307,34 @@ BH_DEV void trace_tile(const TraceParams& P, unsigned tile, unsigned lane, unsig
         live = (st == RAY_LIVE);
         fin = (st == RAY_DONE);
     }
-    while (live)
-        if (ray.advance(P)) { live = false; fin = true; }
-    __syncwarp();
+    if constexpr (Ray::kParks)
+    {   // A passage is some dozen FP64 steps, and the lanes of a tile come to the cap at different
+        // steps; one lane's passage would keep the others waiting.  So a lane waits at the cap
+        // until the others have come to it or ended (or for kCapWait steps, which bounds the
+        // wait for a lane near the photon sphere), and the waiting ones pass together.
+        // Near-extremal sweep, 4K at 45 deg: 52.3 ms before, 36.4 ms so; 1080p at 88.9 deg:
+        // 43.8 ms, 16.4 ms.  (Waits of at most 32 / 64 / 128 / 256 steps: 43.3 / 38.7 / 36.8 /
+        // 36.6 and 33.5 / 26.0 / 20.5 / 17.8 ms.)
+        constexpr int kCapWait = 512;
+        while (__any_sync(0xffffffffu, live))
+        {
+            bool waits = false;
+            for (int n = 0; live && !waits && n < kCapWait; ++n)
+            {
+                if (ray.advance(P)) { live = false; fin = true; }
+                else waits = ray.parked;
+            }
+            __syncwarp();
+            if (waits && pass_cap(P, ray)) { live = false; fin = true; }
+            __syncwarp();
+        }
+    }
+    else
+    {
+        while (live)
+            if (ray.advance(P)) { live = false; fin = true; }
+        __syncwarp();
+    }
     if (fin)
     {
         PackedRay<typename Ray::Real> q;

@@ -36,3 +36,18 @@ def test_step_forms_match_oracle(cuda, oracle, case, disk):
     s = parity.compare_rays(probe_grid(P, NX, NY), oracle.probe_grid(P, NX, NY))
     assert s["cls_mismatch_inner"] == 0, s
     assert s["esc_frac_1e4"] >= share, s
+
+
+@pytest.mark.parametrize("steps", [24, 37, 2000])
+def test_mixed_passages_match_fp64(cuda, steps):
+    """FP64 polar passages taken together by a warp's lanes, with step budgets that end
+    inside a passage or just after it, against the all-FP64 integration."""
+    from bhrt.device import probe_grid
+    P = scenes.scene(lib.derive, BH_KERR, 0.9, 0.0, NX, NY, 12.0, 89.5, 50.0)
+    P.maxSteps = steps
+    got, want = probe_grid(P, NX, NY, precision=1), probe_grid(P, NX, NY, precision=2)
+    s = parity.compare_rays(got, want)
+    assert s["outcome_mismatch_inner"] == 0, s
+    assert s["esc_frac_1e4"] >= 0.98, s
+    again = probe_grid(P, NX, NY, precision=1)
+    assert again.tobytes() == got.tobytes()
