@@ -514,6 +514,7 @@ cudaError_t bhSurrogateCreate(BHSurrogate** out, unsigned seed)
     if (e == cudaSuccess) e = bh_tc_error_word(&S.err);
     // every set-up write goes on the network's stream, ordered with the kernels that follow
     if (e == cudaSuccess) e = cudaMemsetAsync(S.W, 0, kWCount * 2, s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S.Wt, 0, kWCount * 2, s->stream);   // the head's padding stays zero
     if (e != cudaSuccess) { freeAll(s); return e; }
     // Xavier-uniform weights, zero biases
     std::vector<float> p(SgLayout::count(), 0.f);
@@ -600,7 +601,7 @@ cudaError_t bhSurrogateForward(BHSurrogate* s, const float* in, float* out, int 
         SgInferArgs a{S.W, S.W + 4 * kHidW, S.biasPacked, in, out, (unsigned)n, S.err};
         return sg_infer_launch(a, nullptr, stream);
     }
-    cudaError_t e = sg_forward_train(S, in, n, stream);
+    cudaError_t e = sg_forward_train(S, in, n, false, stream);
     if (e != cudaSuccess) return e;
     return cudaMemcpyAsync(out, S.Y, (size_t)n * 16 * sizeof(float), cudaMemcpyDeviceToDevice, stream);
 }
@@ -612,7 +613,8 @@ cudaError_t bhSurrogateGradients(BHSurrogate* s, const float* in, const float* t
     SgState& S = s->S;
     // the caller's inputs may come from any stream: wait for all prior work
     cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = sg_gradients(S, in, tgt, n, s->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S.loss, 0, 8 * sizeof(float), s->stream);
+    if (e == cudaSuccess) e = sg_gradients(S, in, tgt, n, S.loss, false, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e == cudaSuccess) e = checkErrWord(s);
     if (e == cudaSuccess && gradsHost)
@@ -772,15 +774,14 @@ cudaError_t bhSurrogateTrain(BHSurrogate* s, int steps, int batch, float lr, uns
     }
     float* hist = nullptr;
     if (steps > 0 && (e = bh_device_alloc(reinterpret_cast<void**>(&hist), (size_t)steps * 8 * sizeof(float))) != cudaSuccess) return e;
+    if (steps > 0) e = cudaMemsetAsync(hist, 0, (size_t)steps * 8 * sizeof(float), s->stream);
     for (int it = 0; it < steps && e == cudaSuccess; ++it)
     {
         const float t = steps > 1 ? (float)it / (float)(steps - 1) : 0.f;
         const float lrT = lr * (0.05f + 0.95f * 0.5f * (1.f + std::cos(kPi * t)));
         e = sg_gather(S, seed * 0x9E3779B1u + (unsigned)it * 0x632BE5ABu, s->bIn, s->bTgt, batch, s->stream);
-        if (e == cudaSuccess) e = sg_gradients(S, s->bIn, s->bTgt, batch, s->stream);
+        if (e == cudaSuccess) e = sg_gradients(S, s->bIn, s->bTgt, batch, hist + (size_t)it * 8, true, s->stream);
         if (e == cudaSuccess) e = sg_adam(S, lrT, s->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(hist + (size_t)it * 8, S.loss, 8 * sizeof(float), cudaMemcpyDeviceToDevice, s->stream);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e == cudaSuccess) e = checkErrWord(s);

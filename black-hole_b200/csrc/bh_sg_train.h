@@ -36,15 +36,10 @@ struct SgState
     // per-batch scratch (capacity `cap` rays)
     int cap = 0;
     void* X[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // BF16 n x 256 activations
-    float* Z[4] = {nullptr, nullptr, nullptr, nullptr};           // FP32 n x 256 pre-activations
+    float* Z[4] = {nullptr, nullptr, nullptr, nullptr};           // FP32 pre-activations, 128-row tiles of [column / 4][row][4]
     float* Y = nullptr;               // FP32 n x 16
     void* dY = nullptr;               // BF16 n x 64
-    void* dYt = nullptr;              // BF16 128 x n (rows >= 16 zero)
-    float* dX = nullptr;              // FP32 n x 256
-    void* dZ = nullptr;               // BF16 n x 256
-    void* T0 = nullptr;               // BF16 256 x n transposes
-    void* T1 = nullptr;
-    float* headTmp = nullptr;         // FP32 128 x 256
+    void* dZ[4] = {nullptr, nullptr, nullptr, nullptr};           // BF16 n x 256
 
     // the RK4-traced ray set: inputs (n x 8) and targets (n x 8)
     float* dsIn = nullptr;
@@ -55,9 +50,18 @@ struct SgState
 cudaError_t sg_features(const float* in, void* X0, int n, cudaStream_t s);
 cudaError_t sg_pack_weights(SgState& S, cudaStream_t s);
 // grows the per-batch scratch to n rays; the zero fill is enqueued on s
-cudaError_t sg_reserve(SgState& S, int n, cudaStream_t s);
+cudaError_t sg_reserve(SgState& S, int n);
 void sg_free_batch(SgState& S);
-cudaError_t sg_forward_train(SgState& S, const float* in, int n, cudaStream_t s);
-cudaError_t sg_gradients(SgState& S, const float* in, const float* tgt, int n, cudaStream_t s);
+cudaError_t sg_forward_train(SgState& S, const float* in, int n, bool haveFeatures, cudaStream_t s);
+// `loss`: 8 floats, zeroed by the caller, that receive the batch's loss sums; with
+// `haveFeatures` S.X[0] holds the features of `in` already
+cudaError_t sg_gradients(SgState& S, const float* in, const float* tgt, int n, float* loss, bool haveFeatures,
+                         cudaStream_t s);
 cudaError_t sg_adam(SgState& S, float lr, cudaStream_t s);
-cudaError_t sg_gather(const SgState& S, unsigned seed, float* in, float* tgt, int n, cudaStream_t s);
+// the training GEMMs with their epilogues (bh_sg_layer.cu): Z_l and X_{l+1} from X_l; dZ_l and
+// the bias gradient from dZ_{l+1} (or dY) and Z_l; all weight gradients, added to S.grads
+cudaError_t sg_layer_forward(const SgState& S, int l, int n, cudaStream_t s);
+cudaError_t sg_layer_backward(const SgState& S, int l, int n, cudaStream_t s);
+cudaError_t sg_weight_grads(const SgState& S, int n, cudaStream_t s);
+// the step's batch: rows of the ray set at hashed indices (in, tgt) and their features (S.X[0])
+cudaError_t sg_gather(SgState& S, unsigned seed, float* in, float* tgt, int n, cudaStream_t s);

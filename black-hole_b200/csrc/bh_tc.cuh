@@ -105,6 +105,21 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, uint64_
         : "memory");
 }
 
+// 2-D tiled store of a box in shared memory to (x, y) >= 0; rows past the tensor are
+// clipped.  The writer's generic stores must have been fenced (fence_async_smem).
+__device__ __forceinline__ void tma_store_2d(const void* tmap, const void* src, int x, int y)
+{
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                 ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(src)), "r"(x), "r"(y) : "memory");
+}
+
+// all stores that this thread issued: done, and their writes visible to later kernels
+__device__ __forceinline__ void tma_store_wait()
+{
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap)
 {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
