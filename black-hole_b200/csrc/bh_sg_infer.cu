@@ -26,6 +26,12 @@
 // (multicast MMA commits to both CTAs), aReady[g] (leader: 512 epilogue
 // arrivals from both CTAs -- the operand of the next layer is in shared memory
 // and the accumulator is free).  All waits are bounded (bh_tc.cuh).
+// Bound: the groups' chain per layer, 2600 cycles of MMA (2048 of them tensor core),
+// four 32-column turns of 840 .. 1200 cycles (tanh: 256 of the special-function unit a
+// warp and turn) and 1000 for the cluster-scope arrival; features 5300 a tile.  All
+// column indexes of the epilogue and the features are constants, accumulators load while
+// the columns before are turned, and a wait reads the timer only after it ran out once:
+// 2,000,003 rays 1.292 -> 1.218 ms (the features' inputs were indexed through local memory).
 // ---------------------------------------------------------------------------
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -54,17 +60,26 @@ struct Bars
     uint32_t tmem;
 };
 
-// 8 packed BF16 values -> the operand row `row`, columns col .. col + 7
-__device__ __forceinline__ void st_chunk(uint8_t* tile, uint32_t row, uint32_t col, uint4 v)
+// 8 packed BF16 values -> columns 8 j .. 8 j + 7 (j a constant) of the operand row at
+// `rowPtr` (sw128_offset(row, 0, 128) on) with `swz` = row % 8
+__device__ __forceinline__ void st_chunk(uint8_t* rowPtr, uint32_t swz, uint32_t j, uint4 v)
 {
-    *reinterpret_cast<uint4*>(tile + sw128_offset(row, col, 128)) = v;
+    *reinterpret_cast<uint4*>(rowPtr + (((j & 7u) ^ swz) << 4) + (j >> 3) * 16384u) = v;
+}
+
+// half of the features of one ray (chunks J0 .. J0 + 15), all indexes constant
+template <int J0>
+__device__ __forceinline__ void st_features(uint8_t* rowPtr, uint32_t swz, const float* x)
+{
+#pragma unroll
+    for (int j = J0; j < J0 + 16; ++j) st_chunk(rowPtr, swz, (uint32_t)j, sg_feature_chunk(x, j));
 }
 
 // (acc + bias) / 2 in one packed FP32 FMA (bias2 = bias / 2; exact halving),
 // BF16 rounding, GELU from the halved input (bit-identical to gelu2)
-__device__ __forceinline__ uint32_t pack_gelu(float a, float b, float ba2, float bb2)
+__device__ __forceinline__ uint32_t pack_gelu(uint32_t a, uint32_t b, float ba2, float bb2)
 {
-    const float2 z = __ffma2_rn(make_float2(a, b), make_float2(0.5f, 0.5f), make_float2(ba2, bb2));
+    const float2 z = __ffma2_rn(make_float2(__uint_as_float(a), __uint_as_float(b)), make_float2(0.5f, 0.5f), make_float2(ba2, bb2));
     __nv_bfloat162 h = gelu2_half(__floats2bfloat162_rn(z.x, z.y));
     return *reinterpret_cast<uint32_t*>(&h);
 }
@@ -284,7 +299,9 @@ sg_infer_kernel(const __grid_constant__ CUtensorMap tW, const __grid_constant__ 
     {   // ---- epilogue groups ----
         const int g = warp >> 3, wq = warp & 3, half = (warp >> 2) & 1;
         const uint32_t row = (uint32_t)(wq * 32 + lane);
-        uint8_t* tile = tiles + g * kTileBytes;
+        const uint32_t swz = row & 7u;
+        uint8_t* rowPtr = tiles + g * kTileBytes + sw128_offset(row, 0, 128) - (swz << 4);
+        uint8_t* halfPtr = rowPtr + half * 32768;             // columns 128 half ..
         const uint32_t tl = tmem + (uint32_t)g * 256u + ((uint32_t)(wq * 32) << 16);
         const uint32_t aReadyLeader = mapa_shared(&B.aReady[g], 0);
         uint32_t phF = 0;
@@ -305,9 +322,8 @@ sg_infer_kernel(const __grid_constant__ CUtensorMap tW, const __grid_constant__ 
 #pragma unroll
                 for (int k = 0; k < kIn; ++k) r.x[k] = valid ? __ldg(rawIn + (size_t)rid * 8 + k) : 0.f;
             }
-#pragma unroll 4
-            for (int j = half * 16; j < half * 16 + 16; ++j)
-                st_chunk(tile, row, (uint32_t)j * 8u, sg_feature_chunk(r.x, j));
+            if (half == 0) st_features<0>(rowPtr, swz, r.x);
+            else st_features<16>(rowPtr, swz, r.x);
             fence_async_smem();
             mbar_arrive_cluster(aReadyLeader);
 
@@ -317,25 +333,31 @@ sg_infer_kernel(const __grid_constant__ CUtensorMap tW, const __grid_constant__ 
                 phF ^= 1u;
                 if (!ok) break;
                 tc_fence_after();
-                const float* bl = sBias + l * kWidth;
-#pragma unroll 1
-                for (int c = half * 128; c < half * 128 + 128; c += 32)
+                // 4 x 32 columns, the next ones on their way from TMEM while these are turned
+                const float* bl = sBias + l * kWidth + half * 128;
+                const uint32_t th = tl + (uint32_t)half * 128u;
+                uint32_t v[2][32];
+                tmem_ld32_start(th, v[0]);
+                tmem_ld32_wait(v[0]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
                 {
-                    float v[32];
-                    tmem_ld32(tl + (uint32_t)c, v);
+                    if (k < 3) tmem_ld32_start(th + (uint32_t)(k + 1) * 32u, v[(k + 1) & 1]);
+                    const uint32_t* u = v[k & 1];
 #pragma unroll
                     for (int q4 = 0; q4 < 4; ++q4)
                     {
                         uint4 o;
-                        const int b = c + q4 * 8;
+                        const int b = k * 32 + q4 * 8;
                         const float4 b0 = *reinterpret_cast<const float4*>(bl + b);
                         const float4 b1 = *reinterpret_cast<const float4*>(bl + b + 4);
-                        o.x = pack_gelu(v[q4 * 8 + 0], v[q4 * 8 + 1], b0.x, b0.y);
-                        o.y = pack_gelu(v[q4 * 8 + 2], v[q4 * 8 + 3], b0.z, b0.w);
-                        o.z = pack_gelu(v[q4 * 8 + 4], v[q4 * 8 + 5], b1.x, b1.y);
-                        o.w = pack_gelu(v[q4 * 8 + 6], v[q4 * 8 + 7], b1.z, b1.w);
-                        st_chunk(tile, row, (uint32_t)b, o);
+                        o.x = pack_gelu(u[q4 * 8 + 0], u[q4 * 8 + 1], b0.x, b0.y);
+                        o.y = pack_gelu(u[q4 * 8 + 2], u[q4 * 8 + 3], b0.z, b0.w);
+                        o.z = pack_gelu(u[q4 * 8 + 4], u[q4 * 8 + 5], b1.x, b1.y);
+                        o.w = pack_gelu(u[q4 * 8 + 6], u[q4 * 8 + 7], b1.z, b1.w);
+                        st_chunk(halfPtr, swz, (uint32_t)(k * 4 + q4), o);
                     }
+                    if (k < 3) tmem_ld32_wait(v[(k + 1) & 1]);
                 }
                 tc_fence_before();
                 fence_async_smem();
