@@ -579,18 +579,38 @@ int rays_per_warp(const TraceParams& P)
     return width;
 }
 
+// Warps an SM of the tile kernel for a middling frame (0: as many as fit).  Up to some tens
+// of thousands of tiles a frame ends with a few warps whose rays go round the hole; those
+// started first and ran all the while next to 25 .. 28 others, so fewer warps an SM let them
+// through sooner (1283 x 719 Reissner-Nordstroem: the queue empty at 1.17 ms, the last warp,
+// begun at 0, at 1.77).  Geometric means over random views, against all that fit:
+// spherical 512 x 288 and 640 x 360 at 12 warps 1.06 .. 1.08x, 960 x 540 at 16 1.03x, 1283 x 719
+// at 20 1.02x (1.05 .. 1.09x where one ray is the frame; never slower), 1920 x 1080 at 24 0.98 .. 1.09 (not taken);
+// rotating 512 x 288 .. 960 x 540 at 15 1.03 .. 1.05x, 1283 x 719 at 20 0.99x (not taken).
+// Fewer still help more at the mean, but cost views without such rays up to 10 %.
+int warps_per_sm(const TraceParams& P, bool kerr)
+{
+    if (P.nRaysDev || P.raysPerWarp < 32) return 0;
+    const unsigned tiles = P.nRays / 32u;
+    if (tiles <= 8192u) return kerr ? 15 : 12;
+    if (tiles <= 16384u) return kerr ? 15 : 16;
+    return tiles <= 32768u && !kerr ? 20 : 0;
+}
+
 template <class Ray, bool STATS>
 cudaError_t launch_one(const TraceParams& P0, int blocksPerSm, cudaStream_t stream)
 {
     TraceParams P = P0;
     P.raysPerWarp = 32;
     auto k = trace_kernel<Ray, STATS>;
+    constexpr int block = block_of<Ray, STATS>();
     if constexpr (!STATS && sizeof(typename Ray::Real) == 4)
     {   // whole frames under the default work distribution: tile-synchronous
         if (P.refillMin >= 32 && !P.dirs)
         {
             k = tile_kernel<Ray>;
             P.raysPerWarp = rays_per_warp(P);
+            if (blocksPerSm == 0) blocksPerSm = warps_per_sm(P, Ray::kKerrFamily) * 32 / block;
         }
     }
     int dev = 0, sms = 0, occ = 0;
@@ -598,7 +618,6 @@ cudaError_t launch_one(const TraceParams& P0, int blocksPerSm, cudaStream_t stre
     if (e != cudaSuccess) return e;
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    constexpr int block = block_of<Ray, STATS>();
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, block, 0);
     if (e != cudaSuccess) return e;
     if (occ < 1) occ = 1;
