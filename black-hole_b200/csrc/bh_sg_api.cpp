@@ -142,10 +142,6 @@ struct BHSurrogate
     cudaEvent_t setDone[2] = {nullptr, nullptr};
     size_t setUnits = 0;
     bool setPinned = false;
-    // batch buffers of the training loop
-    float* bIn = nullptr;
-    float* bTgt = nullptr;
-    int bCap = 0;
     // anchored frames: RK4 anchors every anchorStride pixels (0: the network's own directions)
     int anchorStride = 8;
     bool anchorNet = true;
@@ -209,7 +205,7 @@ void freeAll(BHSurrogate* s)
     SgState& S = s->S;
     sg_free_batch(S);
     void* ps[] = {S.params, S.grads, S.adamM, S.adamV, S.W, S.Wt, S.biasPacked, S.loss, S.dsIn, S.dsTgt, s->list,
-                  s->counters, s->heldPix, s->heldPred, s->bIn, s->bTgt, s->anchorPix, s->anchorRecIdx, s->anchorRec,
+                  s->counters, s->heldPix, s->heldPred, s->anchorPix, s->anchorRecIdx, s->anchorRec,
                   s->cellPix, s->cellGate, s->sampleDir, s->samplePix, s->blockOrder};
     for (void* p : ps)
         if (p) cudaFree(p);
@@ -601,9 +597,7 @@ cudaError_t bhSurrogateForward(BHSurrogate* s, const float* in, float* out, int 
         SgInferArgs a{S.W, S.W + 4 * kHidW, S.biasPacked, in, out, (unsigned)n, S.err};
         return sg_infer_launch(a, nullptr, stream);
     }
-    cudaError_t e = sg_forward_train(S, in, n, false, stream);
-    if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(out, S.Y, (size_t)n * 16 * sizeof(float), cudaMemcpyDeviceToDevice, stream);
+    return sg_chain_forward(S, in, out, n, stream);
 }
 
 cudaError_t bhSurrogateGradients(BHSurrogate* s, const float* in, const float* tgt, int n, float* gradsHost,
@@ -614,7 +608,7 @@ cudaError_t bhSurrogateGradients(BHSurrogate* s, const float* in, const float* t
     // the caller's inputs may come from any stream: wait for all prior work
     cudaError_t e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = cudaMemsetAsync(S.loss, 0, 8 * sizeof(float), s->stream);
-    if (e == cudaSuccess) e = sg_gradients(S, in, tgt, n, S.loss, false, s->stream);
+    if (e == cudaSuccess) e = sg_gradients(S, in, tgt, 0, 0u, n, S.loss, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e == cudaSuccess) e = checkErrWord(s);
     if (e == cudaSuccess && gradsHost)
@@ -762,16 +756,6 @@ cudaError_t bhSurrogateTrain(BHSurrogate* s, int steps, int batch, float lr, uns
     SgState& S = s->S;
     if (S.dsN <= 0) return cudaErrorInvalidValue;
     cudaError_t e = cudaSuccess;
-    if (batch > s->bCap)
-    {
-        if (s->bIn) cudaFree(s->bIn);
-        if (s->bTgt) cudaFree(s->bTgt);
-        s->bIn = s->bTgt = nullptr;
-        s->bCap = 0;
-        if ((e = bh_device_alloc(reinterpret_cast<void**>(&s->bIn), (size_t)batch * 8 * sizeof(float))) != cudaSuccess) return e;
-        if ((e = bh_device_alloc(reinterpret_cast<void**>(&s->bTgt), (size_t)batch * 8 * sizeof(float))) != cudaSuccess) return e;
-        s->bCap = batch;
-    }
     float* hist = nullptr;
     if (steps > 0 && (e = bh_device_alloc(reinterpret_cast<void**>(&hist), (size_t)steps * 8 * sizeof(float))) != cudaSuccess) return e;
     if (steps > 0) e = cudaMemsetAsync(hist, 0, (size_t)steps * 8 * sizeof(float), s->stream);
@@ -779,8 +763,8 @@ cudaError_t bhSurrogateTrain(BHSurrogate* s, int steps, int batch, float lr, uns
     {
         const float t = steps > 1 ? (float)it / (float)(steps - 1) : 0.f;
         const float lrT = lr * (0.05f + 0.95f * 0.5f * (1.f + std::cos(kPi * t)));
-        e = sg_gather(S, seed * 0x9E3779B1u + (unsigned)it * 0x632BE5ABu, s->bIn, s->bTgt, batch, s->stream);
-        if (e == cudaSuccess) e = sg_gradients(S, s->bIn, s->bTgt, batch, hist + (size_t)it * 8, true, s->stream);
+        e = sg_gradients(S, S.dsIn, S.dsTgt, S.dsN, seed * 0x9E3779B1u + (unsigned)it * 0x632BE5ABu, batch,
+                         hist + (size_t)it * 8, s->stream);
         if (e == cudaSuccess) e = sg_adam(S, lrT, s->stream);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);

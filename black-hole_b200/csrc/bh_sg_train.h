@@ -37,7 +37,6 @@ struct SgState
     int cap = 0;
     void* X[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // BF16 n x 256 activations
     float* Z[4] = {nullptr, nullptr, nullptr, nullptr};           // FP32 pre-activations, 128-row tiles of [column / 4][row][4]
-    float* Y = nullptr;               // FP32 n x 16
     void* dY = nullptr;               // BF16 n x 64
     void* dZ[4] = {nullptr, nullptr, nullptr, nullptr};           // BF16 n x 256
 
@@ -49,19 +48,17 @@ struct SgState
 
 cudaError_t sg_features(const float* in, void* X0, int n, cudaStream_t s);
 cudaError_t sg_pack_weights(SgState& S, cudaStream_t s);
-// grows the per-batch scratch to n rays; the zero fill is enqueued on s
+// grows the per-batch scratch to n rays
 cudaError_t sg_reserve(SgState& S, int n);
 void sg_free_batch(SgState& S);
-cudaError_t sg_forward_train(SgState& S, const float* in, int n, bool haveFeatures, cudaStream_t s);
-// `loss`: 8 floats, zeroed by the caller, that receive the batch's loss sums; with
-// `haveFeatures` S.X[0] holds the features of `in` already
-cudaError_t sg_gradients(SgState& S, const float* in, const float* tgt, int n, float* loss, bool haveFeatures,
+// Forward, loss and backward of n rays; `loss`: 8 floats, zeroed by the caller, that receive
+// the batch's loss sums.  N > 0: the batch is rows of in / tgt at hashed indices below N.
+cudaError_t sg_gradients(SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n, float* loss,
                          cudaStream_t s);
 cudaError_t sg_adam(SgState& S, float lr, cudaStream_t s);
-// the training GEMMs with their epilogues (bh_sg_layer.cu): Z_l and X_{l+1} from X_l; dZ_l and
-// the bias gradient from dZ_{l+1} (or dY) and Z_l; all weight gradients, added to S.grads
-cudaError_t sg_layer_forward(const SgState& S, int l, int n, cudaStream_t s);
-cudaError_t sg_layer_backward(const SgState& S, int l, int n, cudaStream_t s);
+// the kernels of bh_sg_chain.cu: Y (n x 16) = net(in) in the training form; its activations, dZ_l
+// and bias gradients; all weight gradients, added to S.grads
+cudaError_t sg_chain_forward(const SgState& S, const float* in, float* Y, int n, cudaStream_t s);
+cudaError_t sg_chain_train(const SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n,
+                           float* loss, cudaStream_t s);
 cudaError_t sg_weight_grads(const SgState& S, int n, cudaStream_t s);
-// the step's batch: rows of the ray set at hashed indices (in, tgt) and their features (S.X[0])
-cudaError_t sg_gather(SgState& S, unsigned seed, float* in, float* tgt, int n, cudaStream_t s);

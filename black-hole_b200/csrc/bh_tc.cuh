@@ -113,12 +113,13 @@ __device__ __forceinline__ void tma_store_2d(const void* tmap, const void* src, 
                  ::"l"(reinterpret_cast<uint64_t>(tmap)), "r"(smem_u32(src)), "r"(x), "r"(y) : "memory");
 }
 
-// all stores that this thread issued: done, and their writes visible to later kernels
-__device__ __forceinline__ void tma_store_wait()
-{
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+
+// the stores that this thread committed: their shared memory is read
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
+// the stores that this thread committed: done, and visible to later kernels
+__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap)
 {
