@@ -1,6 +1,6 @@
 // ---------------------------------------------------------------------------
 // bh_gemm.cu -- BF16 tensor-core GEMM with FP32 accumulation (tcgen05 + TMA),
-// the workhorse of the surrogate's training passes:
+// the general product behind bhTcGemm:
 //
 //     C[M x N] (=|+=) A[M x K] . B[N x K]^T (+ bias[N])
 //

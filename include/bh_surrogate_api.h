@@ -88,7 +88,7 @@ cudaError_t bhSurrogateFeatures(const float* in, void* features, int n, cudaStre
 
 /* Head outputs (n x 16 floats) of n input rows.  fused != 0: the fused
  * persistent tensor-core kernel used for rendering; fused == 0: the training
- * path (one tensor-core GEMM per layer plus element-wise kernels). */
+ * form (the kernel of the training passes, without their stores). */
 cudaError_t bhSurrogateForward(BHSurrogate* s, const float* in, float* out, int n, int fused, cudaStream_t stream);
 
 /* Forward, loss and backward on n rays (n a multiple of 128; device inputs
