@@ -92,11 +92,12 @@ cudaError_t launchPlan(const Plan& pl, const BHView* views, const TraceParams* d
     int blocksK = 0, blocksS = 0;
     bhGetTuning(1, nullptr, &blocksK);
     bhGetTuning(0, nullptr, &blocksS);
-    cudaError_t e = cudaSuccess;
-    if (nK > 0 && (e = bh_launch_batch(true, dTable, dBase, nK, pl.base[nK], counter, blocksK, s)) != cudaSuccess)
+    cudaError_t e = cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned), s);     // one counter a family
+    if (e != cudaSuccess) return e;
+    if (nK > 0 && (e = bh_launch_batch(true, dTable, dBase, nK, pl.base[nK], counter, blocksK, false, s)) != cudaSuccess)
         return e;
-    if (nS > 0 && (e = bh_launch_batch(false, dTable + nK, dBase + nK + 1, nS, pl.base[n + 1], counter, blocksS,
-                                       s)) != cudaSuccess)
+    if (nS > 0 && (e = bh_launch_batch(false, dTable + nK, dBase + nK + 1, nS, pl.base[n + 1], counter + 1, blocksS,
+                                       nK > 0, s)) != cudaSuccess)
         return e;
     for (int i = 0; i < n; ++i)
     {

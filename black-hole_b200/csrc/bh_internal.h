@@ -30,11 +30,13 @@ cudaError_t bh_launch_trace(const TraceParams& P, int precision, bool stats, int
                             cudaStream_t stream);
 
 // batched views of one metric family (`kerr`: Kerr / Kerr-Newman, else the
-// spherical metrics): zero the counter, then one persistent launch over all
-// the views' tiles (bh_trace.cu); `views` and `tileBase` (n + 1 prefix sums of
-// tiles) are device tables
+// spherical metrics): one persistent launch over all the views' tiles
+// (bh_trace.cu); `views` and `tileBase` (n + 1 prefix sums of tiles) are device
+// tables, `counter` is zero.  `beside`: the launch before it on the stream is the other
+// family's, and it starts in that one's tail.
 cudaError_t bh_launch_batch(bool kerr, const TraceParams* views, const unsigned* tileBase, int n,
-                            unsigned totalTiles, unsigned* counter, int blocksPerSm, cudaStream_t stream);
+                            unsigned totalTiles, unsigned* counter, int blocksPerSm, bool beside,
+                            cudaStream_t stream);
 
 // ray sets (bh_trace.cu): sort the rays of the units for tracing, then trace the
 // units of one metric family and write their inputs' targets (bh_sg_train.h)

@@ -382,6 +382,8 @@ batch_kernel(const TraceParams* __restrict__ views, const unsigned* __restrict__
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
     int cur = -1;
+    // the other family's launch may start as soon as SMs are free of this one (bh_launch_batch)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     while (true)
     {
         unsigned g = 0;
@@ -405,6 +407,8 @@ batch_kernel(const TraceParams* __restrict__ views, const unsigned* __restrict__
         trace_tile<Ray>(sp[warp], g - __ldg(tileBase + lo), lane, sp[warp].nRays, 32u);
         __syncwarp();
     }
+    // what follows on the stream needs both families' frames
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 static_assert(sizeof(TraceParams) % 8 == 0, "TraceParams is copied in 8-byte words");
 
@@ -662,11 +666,17 @@ cudaError_t bh_launch_trace(const TraceParams& P, int precision, bool stats, int
                  : launch_one<SphRay<float, false>, false>(P, blocksPerSm, stream);
 }
 
+// A launch ends with a few warps' long rays on a mostly idle GPU (48 views: 1.1 ms of the rotating
+// family's 31.9), and the families share nothing but their place on the stream: the second
+// one takes the SMs that the first has left (programmatic launch: every CTA of the first is
+// running by then, and every CTA of the second waits for the first to end before it ends).
+// 48 views: 44.03 -> 43.28 ms.
 cudaError_t bh_launch_batch(bool kerr, const TraceParams* views, const unsigned* tileBase, int n,
-                            unsigned totalTiles, unsigned* counter, int blocksPerSm, cudaStream_t stream)
+                            unsigned totalTiles, unsigned* counter, int blocksPerSm, bool beside,
+                            cudaStream_t stream)
 {
-    cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned), stream);
-    if (e != cudaSuccess || totalTiles == 0) return e;
+    cudaError_t e = cudaSuccess;
+    if (totalTiles == 0) return e;
     auto k = kerr ? batch_kernel<KerrRay<float, false>> : batch_kernel<SphRay<float, false>>;
     int dev = 0, sms = 0, occ = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
@@ -678,8 +688,16 @@ cudaError_t bh_launch_batch(bool kerr, const TraceParams* views, const unsigned*
     long long grid = (long long)per * sms;
     const long long need = ((long long)totalTiles * 32 + block - 1) / block;
     if (grid > need) grid = need;
-    k<<<(unsigned)grid, block, 0, stream>>>(views, tileBase, n, totalTiles, counter);
-    return cudaGetLastError();
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = beside ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k, views, tileBase, n, totalTiles, counter);
 }
 
 cudaError_t bh_sort_ray_set(const RaySet& S, cudaStream_t stream)
