@@ -213,16 +213,10 @@ chain_kernel(const __grid_constant__ ChainMaps M, const __grid_constant__ ChainA
         for (int k = 0; k < 4; ++k) mbar_init(&full[k], 1);
         mbar_init(&done, 1);
         fence_barrier_init();
-        chain_load(M, 0, weights, full);
     }
     __syncwarp();
+    if (TRAIN) launch_dependents();
     if (warp == 0) tmem_alloc(&tmemSlot, 512);
-    for (int i = threadIdx.x; i < kHidden * kWidth + kOut; i += kChainThreads)
-    {
-        const int l = min(i / kWidth, kHidden);
-        sBias[i] = A.params[SgLayout::b(l) + i - l * kWidth];
-        if (TRAIN && i < kHidden * kWidth) sDb[i] = 0.f;
-    }
 
     // warp w: rows 32 (w % 4) .., columns kChainCols (w / 4) ..
     const int r = (warp & 3) * 32 + lane, c0 = (warp >> 2) * kChainCols;
@@ -239,6 +233,15 @@ chain_kernel(const __grid_constant__ ChainMaps M, const __grid_constant__ ChainA
             case 2: st_features<16>(tile, (uint32_t)r, x); break;
             default: st_features<24>(tile, (uint32_t)r, x); break;
         }
+    }
+    // so far nothing of the step before: its weights, gradients and buffers from here on
+    if (TRAIN) wait_for_previous();
+    if (threadIdx.x == 0) chain_load(M, 0, weights, full);
+    for (int i = threadIdx.x; i < kHidden * kWidth + kOut; i += kChainThreads)
+    {
+        const int l = min(i / kWidth, kHidden);
+        sBias[i] = A.params[SgLayout::b(l) + i - l * kWidth];
+        if (TRAIN && i < kHidden * kWidth) sDb[i] = 0.f;
     }
     fence_async_smem();
     tc_fence_before();
@@ -449,10 +452,12 @@ weight_grad_kernel(const __grid_constant__ GradMaps maps, float* __restrict__ gr
         tma_prefetch_desc(tB);
     }
     __syncwarp();
+    launch_dependents();
     if (warp == 0) tmem_alloc(&tmemSlot, 256);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    wait_for_previous();
     const uint32_t tmem = tmemSlot;
     const int blocks = kb1 - kb0;
 
@@ -524,7 +529,7 @@ weight_grad_kernel(const __grid_constant__ GradMaps maps, float* __restrict__ gr
 }
 
 template <bool TRAIN>
-cudaError_t launch_chain(const SgState& S, ChainArgs& A, cudaStream_t s)
+cudaError_t launch_chain(const SgState& S, ChainArgs& A, bool early, cudaStream_t s)
 {
     ChainMaps M{};
     const __nv_bfloat16* head = S.W + (size_t)kHidden * kWidth * kWidth;
@@ -544,8 +549,7 @@ cudaError_t launch_chain(const SgState& S, ChainArgs& A, cudaStream_t s)
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(chain_kernel<TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmem);
     if (e != cudaSuccess) return e;
-    chain_kernel<TRAIN><<<(A.n + 127) / 128, kChainThreads, kChainSmem, s>>>(M, A);
-    return cudaGetLastError();
+    return sg_launch(chain_kernel<TRAIN>, dim3((A.n + 127) / 128), kChainThreads, kChainSmem, early, s, M, A);
 }
 
 }  // namespace
@@ -556,11 +560,11 @@ cudaError_t sg_chain_forward(const SgState& S, const float* in, float* Y, int n,
     A.in = in;
     A.Y = Y;
     A.n = n;
-    return launch_chain<false>(S, A, s);
+    return launch_chain<false>(S, A, false, s);
 }
 
 cudaError_t sg_chain_train(const SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n,
-                           float* loss, cudaStream_t s)
+                           float* loss, bool early, cudaStream_t s)
 {
     ChainArgs A{};
     A.in = in;
@@ -572,7 +576,7 @@ cudaError_t sg_chain_train(const SgState& S, const float* in, const float* tgt, 
     A.loss = loss;
     A.wEsc = S.wEsc; A.wDiskR = S.wDiskR; A.wDiskG = S.wDiskG; A.wConf = S.wConf; A.escTol = S.escTol;
     A.n = n;
-    return launch_chain<true>(S, A, s);
+    return launch_chain<true>(S, A, early, s);
 }
 
 cudaError_t sg_weight_grads(const SgState& S, int n, cudaStream_t s)
@@ -592,6 +596,5 @@ cudaError_t sg_weight_grads(const SgState& S, int n, cudaStream_t s)
     if (e != cudaSuccess) return e;
     // ten tiles, the batch cut so that all CTAs of the 148 SMs run at once
     const int kBlocks = n / 64, splits = kBlocks < 14 ? kBlocks : 14;
-    weight_grad_kernel<<<dim3(2 * kLayers, splits), 128, kGradSmem, s>>>(maps, S.grads, kBlocks, S.err);
-    return cudaGetLastError();
+    return sg_launch(weight_grad_kernel, dim3(2 * kLayers, splits), 128, kGradSmem, true, s, maps, S.grads, kBlocks, S.err);
 }

@@ -18,6 +18,25 @@ struct SgLayout
     static constexpr __host__ __device__ int count() { return 4 * kHid + 16 * 256 + 16; }
 };
 
+// A launch; `early`: a programmatic one, whose CTAs may start before the kernel launched before it
+// on the stream has ended (a step's three launches wait for one another inside the kernels)
+template <class... P, class... A>
+inline cudaError_t sg_launch(void (*kernel)(P...), dim3 grid, int threads, size_t smem, bool early, cudaStream_t s,
+                             A&&... args)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 struct SgState
 {
     int device = 0;
@@ -51,14 +70,16 @@ cudaError_t sg_pack_weights(SgState& S, cudaStream_t s);
 // grows the per-batch scratch to n rays
 cudaError_t sg_reserve(SgState& S, int n);
 void sg_free_batch(SgState& S);
-// Forward, loss and backward of n rays; `loss`: 8 floats, zeroed by the caller, that receive
-// the batch's loss sums.  N > 0: the batch is rows of in / tgt at hashed indices below N.
+// Forward, loss and backward of n rays, added to S.grads; `loss`: 8 floats that receive the
+// batch's loss sums (the caller zeroes both).  N > 0: the batch is rows of in / tgt at hashed
+// indices below N.  `early`: the launch before it on the stream is sg_adam's.
 cudaError_t sg_gradients(SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n, float* loss,
-                         cudaStream_t s);
+                         bool early, cudaStream_t s);
+// right after sg_gradients; leaves S.grads zero
 cudaError_t sg_adam(SgState& S, float lr, cudaStream_t s);
 // the kernels of bh_sg_chain.cu: Y (n x 16) = net(in) in the training form; its activations, dZ_l
 // and bias gradients; all weight gradients, added to S.grads
 cudaError_t sg_chain_forward(const SgState& S, const float* in, float* Y, int n, cudaStream_t s);
 cudaError_t sg_chain_train(const SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n,
-                           float* loss, cudaStream_t s);
+                           float* loss, bool early, cudaStream_t s);
 cudaError_t sg_weight_grads(const SgState& S, int n, cudaStream_t s);

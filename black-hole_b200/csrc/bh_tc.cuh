@@ -23,6 +23,13 @@
 
 namespace bhtc {
 
+// ---- programmatic launches ----------------------------------------------------
+// The next launch on the stream may start its CTAs (no effect if it is an ordinary one) ...
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ... and waits here for the launch before it to end, its writes visible.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- shared-memory addresses and barriers -----------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
 {
