@@ -588,18 +588,18 @@ int rays_per_warp(const TraceParams& P)
 // started first and ran all the while next to 25 .. 28 others, so fewer warps an SM let them
 // through sooner (1283 x 719 Reissner-Nordstroem: the queue empty at 1.17 ms, the last warp,
 // begun at 0, at 1.77).  Geometric means over random views, against all that fit:
-// 96 x 54 to 320 x 180 at 8 (spherical) 1.08 .. 1.14x and 10 (rotating) 1.05 .. 1.10x (no view
-// slower; 12 and 15 warps 1.00 .. 1.08x), 480 x 270 at 12 1.03x (8: 0.82x for a view) and 10
-// 1.09x; spherical 512 x 288 and 640 x 360 at 12 warps 1.06 .. 1.08x, 960 x 540 at 16 1.03x, 1283 x 719
-// at 20 1.02x (1.05 .. 1.09x where one ray is the frame; never slower), 1920 x 1080 at 24 0.98 .. 1.09 (not taken);
-// rotating 512 x 288 .. 960 x 540 at 15 1.03 .. 1.05x, 1283 x 719 at 20 0.99x (not taken).
-// Fewer still help more at the mean, but cost views without such rays up to 10 %.
+// spherical 96 x 54 to 480 x 270 at 12 warps 1.03 .. 1.08x (8: 1.08 .. 1.14x, but 0.77 .. 0.94x for
+// views that the hole fills), 512 x 288 and 640 x 360 at 12 1.06 .. 1.08x, 960 x 540 at 16 1.03x,
+// 1283 x 719 at 20 1.02x (1.05 .. 1.09x where one ray is the frame), 1920 x 1080 at 24 0.98 ..
+// 1.09x (not taken); rotating up to 160 x 90 at 10 1.07 .. 1.10x (15: 1.04 .. 1.06x), 240 x 135 to
+// 480 x 270 at 15 1.04 .. 1.11x (10: 1.01 .. 1.06x), 512 x 288 .. 960 x 540 at 15 1.03 .. 1.05x,
+// 1283 x 719 at 20 0.99x (not taken).  Fewer still help more at the mean, but cost views without
+// such rays up to 20 %.
 int warps_per_sm(const TraceParams& P, bool kerr)
 {
     if (P.nRaysDev) return 0;
     const unsigned tiles = P.nRays / 32u;
-    if (tiles <= 2048u) return kerr ? 10 : 8;
-    if (tiles <= 4096u) return kerr ? 10 : 12;
+    if (tiles <= 512u && kerr) return 10;
     if (tiles <= 8192u) return kerr ? 15 : 12;
     if (tiles <= 16384u) return kerr ? 15 : 16;
     return tiles <= 32768u && !kerr ? 20 : 0;

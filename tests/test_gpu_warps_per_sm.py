@@ -9,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("family,model,a", [(0, BH_REISSNER_NORDSTROM, 0.0), (1, BH_KERR_NEWMAN, 0.7)])
-@pytest.mark.parametrize("size", [(320, 200), (328, 200), (512, 256), (520, 256), (1024, 256), (1032, 256), (1024, 512), (1031, 515), (2048, 512), (2056, 512)])
+@pytest.mark.parametrize("size", [(128, 128), (136, 128), (512, 256), (520, 256), (1024, 256), (1032, 256), (1024, 512), (1031, 515), (2048, 512), (2056, 512)])
 def test_frame_does_not_depend_on_blocks_per_sm(cuda, family, model, a, size):
     import torch
     from bhrt.device import Frame
