@@ -607,9 +607,8 @@ cudaError_t bhSurrogateGradients(BHSurrogate* s, const float* in, const float* t
     SgState& S = s->S;
     // the caller's inputs may come from any stream: wait for all prior work
     cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemsetAsync(S.loss, 0, 8 * sizeof(float), s->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(S.grads, 0, SgLayout::count() * sizeof(float), s->stream);
-    if (e == cudaSuccess) e = sg_gradients(S, in, tgt, 0, 0u, n, S.loss, false, s->stream);
+    if (e == cudaSuccess) e = sg_backward(S, in, tgt, 0, 0u, n, false, s->stream);
+    if (e == cudaSuccess) e = sg_gradients(S, n, S.loss, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e == cudaSuccess) e = checkErrWord(s);
     if (e == cudaSuccess && gradsHost)
@@ -759,15 +758,13 @@ cudaError_t bhSurrogateTrain(BHSurrogate* s, int steps, int batch, float lr, uns
     cudaError_t e = cudaSuccess;
     float* hist = nullptr;
     if (steps > 0 && (e = bh_device_alloc(reinterpret_cast<void**>(&hist), (size_t)steps * 8 * sizeof(float))) != cudaSuccess) return e;
-    if (steps > 0) e = cudaMemsetAsync(hist, 0, (size_t)steps * 8 * sizeof(float), s->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(S.grads, 0, SgLayout::count() * sizeof(float), s->stream);
     for (int it = 0; it < steps && e == cudaSuccess; ++it)
     {
         const float t = steps > 1 ? (float)it / (float)(steps - 1) : 0.f;
         const float lrT = lr * (0.05f + 0.95f * 0.5f * (1.f + std::cos(kPi * t)));
-        e = sg_gradients(S, S.dsIn, S.dsTgt, S.dsN, seed * 0x9E3779B1u + (unsigned)it * 0x632BE5ABu, batch,
-                         hist + (size_t)it * 8, it > 0, s->stream);
-        if (e == cudaSuccess) e = sg_adam(S, lrT, s->stream);
+        e = sg_backward(S, S.dsIn, S.dsTgt, S.dsN, seed * 0x9E3779B1u + (unsigned)it * 0x632BE5ABu, batch, it > 0,
+                        s->stream);
+        if (e == cudaSuccess) e = sg_adam(S, batch, lrT, hist + (size_t)it * 8, s->stream);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e == cudaSuccess) e = checkErrWord(s);

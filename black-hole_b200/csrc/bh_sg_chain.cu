@@ -4,7 +4,9 @@
 //   chain_kernel        features, four layers, head (and loss, and the way back):
 //                       Z_l = X_l W_l^T + b_l,  X_{l+1} = gelu(Z_l),  Y = X_4 Wh^T + bh,
 //                       dY,  dZ_l = (dZ_{l+1} W_{l+1}) * gelu'(Z_l),  db_l
-//   weight_grad_kernel  dW_l += dZ_l^T X_l of every layer and the head
+//   weight_grad_kernel  dW_l = dZ_l^T X_l of every layer and the head
+//
+// All sums over the batch are added in a fixed order (bh_sg_train.h), so a step repeats bit for bit.
 //
 // chain_kernel: a ray's passes need no other ray, so one CTA takes 128 rays all the way.
 // Its 128 x 256 BF16 operand stays in shared memory and each layer's result takes its place
@@ -21,9 +23,11 @@
 // weight_grad_kernel: the contraction runs over the rows of the batch, so both
 // operands are read as they lie, with the contraction index as the outer one
 // (MN-major descriptors), instead of through transposed copies.  One launch for
-// all five products: a CTA takes one 128-row tile of one product over a share of the
-// batch and adds it to the gradient with 16-byte reductions.  16,384 rows: 20.7 us
-// (26.6 + 4 x 31 us a product at a time, and ten transposes of 12.4).
+// all five products: a CTA takes one 128-row tile of one product over one part of the
+// batch, an accumulator per share of it.  An accumulator's error grows with its rows (against FP64 over the
+// same BF16 operands 5.0e-7 to 5.6e-7 with shares of 512, 1.1e-6 to 1.3e-6 with 14 of 1,170).  16,384 rows:
+// 24 us (20.7 us with those 14, added by reductions in an order that changed from run to run; 26.6 + 4 x 31 us
+// a product at a time, and ten transposes of 12.4).
 // ---------------------------------------------------------------------------
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -77,7 +81,7 @@ struct ChainArgs
     unsigned seed;
     const float* params;
     float4* Z[kHidden];           // 128-row tiles of [column / 4][row]
-    float *grads, *loss, *Y;
+    float *slices, *Y;
     float wEsc, wDiskR, wDiskG, wConf, escTol;
     int n;
     unsigned* err;
@@ -108,9 +112,9 @@ __device__ __forceinline__ void st_features(uint8_t* tile, uint32_t r, const flo
 }
 
 // Loss terms of one ray from its outputs y; its dY (times 1/n) to row r of the operand.
-// Per warp: loss[0..4] += CE, escape, disk r, disk g, confidence (sums); dbh += column sums of dY.
-__device__ __forceinline__ void chain_loss(const ChainArgs& A, const float* y, const float* x, const float* t,
-                                           uint8_t* tile, uint32_t r)
+// Returns a warp sum a lane: 0..15 the columns of dY, then CE, escape, disk r, disk g, confidence.
+__device__ __forceinline__ float chain_loss(const ChainArgs& A, const float* y, const float* x, const float* t,
+                                            uint8_t* tile, uint32_t r)
 {
     float g[kOut], l[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -160,10 +164,7 @@ __device__ __forceinline__ void chain_loss(const ChainArgs& A, const float* y, c
     float v[32];
 #pragma unroll
     for (int k = 0; k < 32; ++k) v[k] = k < kOut ? g[k] : k < kOut + 5 ? l[k - kOut] : 0.f;
-    const float sum = column_sum(v);
-    const int lane = threadIdx.x & 31;
-    if (lane < kOut + 5 && sum != 0.f)
-        atomicAdd(lane < kOut ? A.grads + SgLayout::b(kHidden) + lane : A.loss + lane - kOut, sum);
+    return column_sum(v);
 }
 
 // 64-column blocks of step s's contraction, and the phase of block kb's barrier in it
@@ -201,7 +202,8 @@ chain_kernel(const __grid_constant__ ChainMaps M, const __grid_constant__ ChainA
     extern __shared__ uint8_t smemRaw[];
     __shared__ uint64_t full[4], done;
     __shared__ uint32_t tmemSlot;
-    __shared__ float sBias[kHidden * kWidth + kOut], sDb[TRAIN ? kHidden * kWidth : 1];
+    // sSum: sums over a warp's 32 rows of dZ_l, dY and the loss terms, a row of them per 32 rays
+    __shared__ float sBias[kHidden * kWidth + kOut], sSum[TRAIN ? 4 : 1][TRAIN ? kSgSlice : 1];
     uint8_t* tile = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
     uint8_t* weights = tile + 4u * kABlock;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -241,7 +243,6 @@ chain_kernel(const __grid_constant__ ChainMaps M, const __grid_constant__ ChainA
     {
         const int l = min(i / kWidth, kHidden);
         sBias[i] = A.params[SgLayout::b(l) + i - l * kWidth];
-        if (TRAIN && i < kHidden * kWidth) sDb[i] = 0.f;
     }
     fence_async_smem();
     tc_fence_before();
@@ -320,7 +321,11 @@ chain_kernel(const __grid_constant__ ChainMaps M, const __grid_constant__ ChainA
                 tmem_ld16(tl + kWidth, y);
 #pragma unroll
                 for (int k = 0; k < kOut; ++k) y[k] += sBias[kHidden * kWidth + k];
-                if constexpr (TRAIN) chain_loss(A, y, x, t, tile, (uint32_t)r);
+                if constexpr (TRAIN)
+                {
+                    const float sum = chain_loss(A, y, x, t, tile, (uint32_t)r);
+                    if (lane < kSgSlice - kHidden * kWidth) sSum[warp][kHidden * kWidth + lane] = sum;
+                }
                 else if (valid)
                 {
 #pragma unroll
@@ -371,11 +376,8 @@ chain_kernel(const __grid_constant__ ChainMaps M, const __grid_constant__ ChainA
                 for (int i = 0; i < 4; ++i)
                     st_operand(tile, (uint32_t)r, (uint32_t)(c / 8 + i),
                                make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]));
-                if (TRAIN && s > kHidden)
-                {
-                    const float sum = column_sum(v);
-                    atomicAdd(&sDb[back * kWidth + c + lane], sum);
-                }
+                if constexpr (TRAIN)
+                    if (s > kHidden) sSum[warp & 3][back * kWidth + c + lane] = column_sum(v);
             }
         }
         fence_async_smem();
@@ -392,15 +394,16 @@ chain_kernel(const __grid_constant__ ChainMaps M, const __grid_constant__ ChainA
     }
     // after a timed-out wait: the CTA leaves only once its copies have landed
     if (!ok && threadIdx.x == 0) chain_landed(loaded, full, A.err);
-    if (TRAIN && ok)
-        for (int i = threadIdx.x; i < kHidden * kWidth; i += kChainThreads)
-            atomicAdd(A.grads + SgLayout::b(i / kWidth) + i % kWidth, sDb[i]);
+    if constexpr (TRAIN)
+        if (ok)
+            for (int i = threadIdx.x; i < kSgSlice; i += kChainThreads)
+                A.slices[(size_t)blockIdx.x * kSgSlice + i] = (sSum[0][i] + sSum[1][i]) + (sSum[2][i] + sSum[3][i]);
     __syncthreads();
     if (warp == 0) tmem_free(tmem, 512);
 }
 
 // ---- weight gradients ----------------------------------------------------------
-constexpr int kGradStages = 4;
+constexpr int kGradStages = 4, kGradThreads = 192;        // four epilogue warps, TMA, MMA
 constexpr uint32_t kBox = 64u * 128u;                     // 64 batch rows x 64 columns
 constexpr uint32_t kGradStage = 6u * kBox;                // 2 boxes of one operand, up to 4 of the other
 constexpr uint32_t kGradSmem = kGradStages * kGradStage + 1024u;
@@ -425,51 +428,57 @@ struct GradMaps
     CUtensorMap cols[kLayers];   // the other one: X_l; dY
 };
 
+// 128-ray tiles of the batch that share k takes start at ...
+__device__ __forceinline__ int share_tile(int tiles, int shares, int k) { return (int)((long long)tiles * k / shares); }
+
 // Tile t = 2 l + h: rows 128 h .. of product l.  The head's is X^T dY (its gradient's transpose).
-__global__ void __launch_bounds__(128, 1)
-weight_grad_kernel(const __grid_constant__ GradMaps maps, float* __restrict__ grads, int kBlocks,
+// blockIdx.y: the part.  Its shares' products go to the two accumulators in turn, so one share is
+// read back and added while the next is multiplied.  The first warps also add the slices of the biases.
+__global__ void __launch_bounds__(kGradThreads, 1)
+weight_grad_kernel(const __grid_constant__ GradMaps maps, const float* slices, float* parts, int tiles,
                    unsigned* __restrict__ err)
 {
     extern __shared__ uint8_t smemRaw[];
-    __shared__ uint64_t full[kGradStages], empty[kGradStages], done;
+    __shared__ uint64_t full[kGradStages], empty[kGradStages], done[2], taken[2];
     __shared__ uint32_t tmemSlot;
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smemRaw) + 1023) & ~uintptr_t(1023));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int l = blockIdx.x >> 1, m0 = (blockIdx.x & 1) * 128;
     const bool head = l == kHidden;
     const int boxes = head ? 1 : 4;                       // 64-column boxes of the second operand
-    const int kb0 = (int)((long long)kBlocks * blockIdx.y / gridDim.y);
-    const int kb1 = (int)((long long)kBlocks * (blockIdx.y + 1) / gridDim.y);
+    const int shares = sg_shares(tiles);
+    const int k0 = shares * (int)blockIdx.y / (int)gridDim.y, k1 = shares * ((int)blockIdx.y + 1) / (int)gridDim.y;
+    float* part = parts + (size_t)blockIdx.y * kSgPart;
     const CUtensorMap* tA = &maps.rows[l];
     const CUtensorMap* tB = &maps.cols[l];
 
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < kGradStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        mbar_init(&done, 1);
+        for (int b = 0; b < 2; ++b) { mbar_init(&done[b], 1); mbar_init(&taken[b], 4); }
         fence_barrier_init();
         tma_prefetch_desc(tA);
         tma_prefetch_desc(tB);
     }
     __syncwarp();
     launch_dependents();
-    if (warp == 0) tmem_alloc(&tmemSlot, 256);
+    if (warp == 0) tmem_alloc(&tmemSlot, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     wait_for_previous();
     const uint32_t tmem = tmemSlot;
-    const int blocks = kb1 - kb0;
 
-    if (threadIdx.x == 0)
+    if (threadIdx.x == 128)
     {
+        const int first = 2 * share_tile(tiles, shares, k0), blocks = 2 * share_tile(tiles, shares, k1) - first;
         int issued = 0;
         for (int kb = 0; kb < blocks; ++kb, ++issued)
         {
             const int s = kb % kGradStages;
             if (kb >= kGradStages && !mbar_wait(&empty[s], ((kb / kGradStages) - 1) & 1, err)) break;
             uint8_t* st = smem + s * kGradStage;
-            const int y = (kb0 + kb) * 64;
+            const int y = (first + kb) * 64;
             mbar_expect_tx(&full[s], (2u + (uint32_t)boxes) * kBox);
             tma_load_2d(st, tA, &full[s], m0, y);
             tma_load_2d(st + kBox, tA, &full[s], m0 + 64, y);
@@ -479,53 +488,80 @@ weight_grad_kernel(const __grid_constant__ GradMaps maps, float* __restrict__ gr
         for (int kb = issued > kGradStages ? issued - kGradStages : 0; kb < issued; ++kb)
             if (!mbar_wait(&full[kb % kGradStages], (kb / kGradStages) & 1, err)) break;
     }
-    else if (threadIdx.x == 32)
+    else if (threadIdx.x == 160)
     {
         const uint32_t idesc = idesc_bf16_f32(head ? 64 : 256) | (1u << 15) | (1u << 16);   // A and B MN-major
-        for (int kb = 0; kb < blocks; ++kb)
+        bool ok = true;
+        int kb = 0;
+        for (int k = k0; k < k1 && ok; ++k)
         {
-            const int s = kb % kGradStages;
-            if (!mbar_wait(&full[s], (kb / kGradStages) & 1, err)) break;
+            const int turn = k - k0, buf = turn & 1;
+            if (turn >= 2 && !mbar_wait(&taken[buf], (uint32_t)((turn >> 1) - 1) & 1u, err)) break;
             tc_fence_after();
-            const uint32_t sa = smem_u32(smem + s * kGradStage), sb = sa + 2u * kBox;
+            const int end = kb + 2 * (share_tile(tiles, shares, k + 1) - share_tile(tiles, shares, k));
+            for (bool more = false; kb < end; ++kb, more = true)
+            {
+                const int s = kb % kGradStages;
+                if (!(ok = mbar_wait(&full[s], (kb / kGradStages) & 1, err))) break;
+                tc_fence_after();
+                const uint32_t sa = smem_u32(smem + s * kGradStage), sb = sa + 2u * kBox;
 #pragma unroll
-            for (int j = 0; j < 4; ++j)      // 16 batch rows each: two atoms on
-                mma_bf16(tmem, sdesc_mn_sw128(sa + j * 2048), sdesc_mn_sw128(sb + j * 2048), idesc, kb > 0 || j > 0);
-            mma_commit(&empty[s]);
+                for (int j = 0; j < 4; ++j)      // 16 batch rows each: two atoms on
+                    mma_bf16(tmem + (uint32_t)buf * 256u, sdesc_mn_sw128(sa + j * 2048), sdesc_mn_sw128(sb + j * 2048),
+                             idesc, more || j > 0);
+                mma_commit(&empty[s]);
+            }
+            mma_commit(&done[buf]);
         }
-        mma_commit(&done);
     }
-    __syncwarp();
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(&done, 0, err));
-    tc_fence_after();
-    if (ok && blocks > 0)
+    else if (warp < 4)
     {
-        const int row = m0 + warp * 32 + lane;
-        const uint32_t tl = tmem + ((uint32_t)(warp * 32) << 16);
-        if (!head)
+        // this tile's biases, one a thread (the head's first tile: its 16 and the loss's 8)
+        if (!head || (m0 == 0 && threadIdx.x < kOut + 8))
         {
-            float* g = grads + SgLayout::w(l) + (size_t)row * kWidth;
+            const float* from = slices + (head ? kHidden * kWidth : l * kWidth + m0) + threadIdx.x;
+            float sum = 0.f;
+            for (int k = k0; k < k1; ++k)
+            {
+                double share = 0.0;
+                const int end = share_tile(tiles, shares, k + 1);
+                for (int t = share_tile(tiles, shares, k); t < end; ++t) share += (double)from[(size_t)t * kSgSlice];
+                sum = k == k0 ? (float)share : sum + (float)share;
+            }
+            part[SgLayout::b(l) + m0 + threadIdx.x] = sum;
+        }
+        __syncwarp();
+        // four columns of a row are a float4, the rows of a tile follow one another (sg_quad).  A float4 is
+        // one thread's: stored with the first share, then added to in the shares' order
+        const uint32_t tl = tmem + ((uint32_t)(warp * 32) << 16);
+        float* g = part + SgLayout::w(l) + m0 * (head ? kOut : kWidth) + 4 * (warp * 32 + lane);
+        for (int k = k0; k < k1; ++k)
+        {
+            const int turn = k - k0, buf = turn & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(&done[buf], (uint32_t)(turn >> 1) & 1u, err))) break;
+            tc_fence_after();
 #pragma unroll 1
-            for (int c = 0; c < kWidth; c += 32)
+            for (int c = 0; c < (head ? kOut : kWidth); c += 16)
             {
                 __syncwarp();
-                float v[32];
-                tmem_ld32(tl + (uint32_t)c, v);
+                float v[16];
+                tmem_ld16(tl + (uint32_t)(buf * 256 + c), v);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) red4(g + c + 4 * i, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                for (int i = 0; i < 4; ++i)
+                {
+                    float* at = g + (c / 4 + i) * 512;
+                    if (turn == 0) *reinterpret_cast<float4*>(at) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    else red4(at, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                }
             }
-        }
-        else
-        {   // row = input unit, column = output unit
-            float v[16];
-            tmem_ld16(tl, v);
-#pragma unroll
-            for (int o = 0; o < kOut; ++o) atomicAdd(grads + SgLayout::w(kHidden) + o * kWidth + row, v[o]);
+            tc_fence_before();
+            if (lane == 0) mbar_arrive(&taken[buf]);
         }
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_free(tmem, 256);
+    if (warp == 0) tmem_free(tmem, 512);
 }
 
 template <bool TRAIN>
@@ -564,7 +600,7 @@ cudaError_t sg_chain_forward(const SgState& S, const float* in, float* Y, int n,
 }
 
 cudaError_t sg_chain_train(const SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n,
-                           float* loss, bool early, cudaStream_t s)
+                           bool early, cudaStream_t s)
 {
     ChainArgs A{};
     A.in = in;
@@ -572,8 +608,7 @@ cudaError_t sg_chain_train(const SgState& S, const float* in, const float* tgt, 
     A.N = N;
     A.seed = seed;
     for (int l = 0; l < kHidden; ++l) A.Z[l] = reinterpret_cast<float4*>(S.Z[l]);
-    A.grads = S.grads;
-    A.loss = loss;
+    A.slices = S.slices;
     A.wEsc = S.wEsc; A.wDiskR = S.wDiskR; A.wDiskG = S.wDiskG; A.wConf = S.wConf; A.escTol = S.escTol;
     A.n = n;
     return launch_chain<true>(S, A, early, s);
@@ -594,7 +629,6 @@ cudaError_t sg_weight_grads(const SgState& S, int n, cudaStream_t s)
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGradSmem);
     if (e != cudaSuccess) return e;
-    // ten tiles, the batch cut so that all CTAs of the 148 SMs run at once
-    const int kBlocks = n / 64, splits = kBlocks < 14 ? kBlocks : 14;
-    return sg_launch(weight_grad_kernel, dim3(2 * kLayers, splits), 128, kGradSmem, true, s, maps, S.grads, kBlocks, S.err);
+    return sg_launch(weight_grad_kernel, dim3(2 * kLayers, sg_parts(n / 128)), kGradThreads, kGradSmem, true, s, maps,
+                     static_cast<const float*>(S.slices), S.parts, n / 128, S.err);
 }

@@ -18,6 +18,17 @@ struct SgLayout
     static constexpr __host__ __device__ int count() { return 4 * kHid + 16 * 256 + 16; }
 };
 
+// What a training step sums over the batch, it sums in a fixed order, so two runs are the same bits:
+// a slice per 128 rays (all biases' gradients and the loss terms); shares of at most four of them (one
+// accumulator of the weight gradients; longer ones only above 64 shares, 32,768 rays); at most 14 parts of
+// some consecutive shares, added in FP32 (ten tiles of products x 14: one CTA an SM); then the parts, in FP64.
+// All by the batch alone, not by the GPU.
+constexpr int kSgBias = 4 * 256 + 16;                       // biases of all layers
+constexpr int kSgSlice = kSgBias + 8;                       // ... and 8 loss terms
+constexpr int kSgPart = SgLayout::count() + 8;              // all gradients and 8 loss terms
+inline __host__ __device__ int sg_shares(int tiles) { return tiles < 4 * 64 ? (tiles + 3) / 4 : 64; }
+inline __host__ __device__ int sg_parts(int tiles) { return sg_shares(tiles) < 14 ? sg_shares(tiles) : 14; }
+
 // A launch; `early`: a programmatic one, whose CTAs may start before the kernel launched before it
 // on the stream has ended (a step's three launches wait for one another inside the kernels)
 template <class... P, class... A>
@@ -47,7 +58,7 @@ struct SgState
     __nv_bfloat16* W = nullptr;       // BF16 W_l (out x in), hidden layers then the 16 x 256 head
     __nv_bfloat16* Wt = nullptr;      // BF16 W_l^T (in x out), hidden layers then the 256 x 64 padded head
     float* biasPacked = nullptr;      // all biases, contiguous (4 x 256 + 16), for the fused kernel
-    float* loss = nullptr;            // 8 floats: loss sums of the last batch
+    float* loss = nullptr;            // 8 floats: loss sums of bhSurrogateGradients' batch
     unsigned* err = nullptr;          // tensor-core kernels' error word
     int step = 0;                     // Adam steps taken
     float wEsc = 100.f, wDiskR = 1.f, wDiskG = 1.f, wConf = 0.1f, escTol = 1e-3f;
@@ -58,6 +69,8 @@ struct SgState
     float* Z[4] = {nullptr, nullptr, nullptr, nullptr};           // FP32 pre-activations, 128-row tiles of [column / 4][row][4]
     void* dY = nullptr;               // BF16 n x 64
     void* dZ[4] = {nullptr, nullptr, nullptr, nullptr};           // BF16 n x 256
+    float* slices = nullptr;          // n / 128 x kSgSlice
+    float* parts = nullptr;           // sg_parts(n / 128) x kSgPart, in groups of four parameters (sg_quad, bh_sg_train.cu)
 
     // the RK4-traced ray set: inputs (n x 8) and targets (n x 8)
     float* dsIn = nullptr;
@@ -70,16 +83,18 @@ cudaError_t sg_pack_weights(SgState& S, cudaStream_t s);
 // grows the per-batch scratch to n rays
 cudaError_t sg_reserve(SgState& S, int n);
 void sg_free_batch(SgState& S);
-// Forward, loss and backward of n rays, added to S.grads; `loss`: 8 floats that receive the
-// batch's loss sums (the caller zeroes both).  N > 0: the batch is rows of in / tgt at hashed
-// indices below N.  `early`: the launch before it on the stream is sg_adam's.
-cudaError_t sg_gradients(SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n, float* loss,
-                         bool early, cudaStream_t s);
-// right after sg_gradients; leaves S.grads zero
-cudaError_t sg_adam(SgState& S, float lr, cudaStream_t s);
+// Forward, loss and backward of n rays; the gradients' parts are left in S.parts.  N > 0: the
+// batch is rows of in / tgt at hashed indices below N.  `early`: the launch before it on the
+// stream is sg_adam's.
+cudaError_t sg_backward(SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n, bool early,
+                        cudaStream_t s);
+// Right after sg_backward of n rays: its loss sums to `loss` (8 floats), and the sums of the
+// gradients to S.grads, or an Adam step with them.
+cudaError_t sg_gradients(SgState& S, int n, float* loss, cudaStream_t s);
+cudaError_t sg_adam(SgState& S, int n, float lr, float* loss, cudaStream_t s);
 // the kernels of bh_sg_chain.cu: Y (n x 16) = net(in) in the training form; its activations, dZ_l
-// and bias gradients; all weight gradients, added to S.grads
+// and slices; the parts of all gradients
 cudaError_t sg_chain_forward(const SgState& S, const float* in, float* Y, int n, cudaStream_t s);
 cudaError_t sg_chain_train(const SgState& S, const float* in, const float* tgt, long long N, unsigned seed, int n,
-                           float* loss, bool early, cudaStream_t s);
+                           bool early, cudaStream_t s);
 cudaError_t sg_weight_grads(const SgState& S, int n, cudaStream_t s);
