@@ -79,8 +79,10 @@ bloom_h_kernel(const float4* __restrict__ acc, float4* __restrict__ hblur, int W
     hblur[(size_t)y * bw + x] = make_float4(rx, ry, rz, 1.f);
 }
 
+// hblur is written while this kernel's first CTAs are there (bh_launch_post), so it is read with
+// ordinary loads behind the wait, neither through __restrict__ nor __ldg; acc was done before.
 __global__ void __launch_bounds__(CP_TX * 4)
-composite_kernel(uchar4* __restrict__ out, const float4* __restrict__ acc, const float4* __restrict__ hblur,
+composite_kernel(uchar4* __restrict__ out, const float4* __restrict__ acc, const float4* hblur,
                  float4* __restrict__ vblur, int W, int H, int bw, int bh, PostConsts pc)
 {
     __shared__ float hs[3][CP_HH][CP_HC];
@@ -96,7 +98,7 @@ composite_kernel(uchar4* __restrict__ out, const float4* __restrict__ acc, const
         {
             int rr = i / CP_HC, cc = i % CP_HC;
             int row = clampi(hr0 - 4 + rr, 0, bh - 1), col = clampi(hc0 + cc, 0, bw - 1);
-            float4 v = __ldg(hblur + (size_t)row * bw + col);
+            float4 v = __ldcg(hblur + (size_t)row * bw + col);
             hs[0][rr][cc] = v.x; hs[1][rr][cc] = v.y; hs[2][rr][cc] = v.z;
         }
         __syncthreads();
