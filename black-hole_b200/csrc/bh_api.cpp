@@ -145,7 +145,7 @@ cudaError_t tileOrder(int W, int H, const unsigned** out)
 struct Tuning
 {
     int refillMin = 32;     // refill a warp when this many lanes are idle
-    int blocksPerSm = 0;    // 0: as many as occupancy allows
+    int blocksPerSm = 0;    // at most so many; 0: as many as fit (small frames: bh_launch_rules.h)
 };
 Tuning gTune[2];            // [0] spherical family, [1] rotating family
 

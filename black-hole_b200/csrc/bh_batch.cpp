@@ -289,6 +289,11 @@ extern "C" void bhBatchGraphDestroy(BHBatchGraph* G)
 // ---------------------------------------------------------------------------
 // autotuner
 // ---------------------------------------------------------------------------
+// The number of CTAs is a limit for all later frames of the family, so it leaves the largest that
+// fit only for a gain beyond the timing's own spread (below the limit of a small frame's rule, all
+// numbers time the same).
+constexpr float kFewer = 0.99f;
+
 extern "C" cudaError_t bhAutotune(const RenderParams& p, int* refillMin, int* blocksPerSm, int* tileOrder,
                                   float* bestMs)
 {
@@ -329,7 +334,7 @@ extern "C" cudaError_t bhAutotune(const RenderParams& p, int* refillMin, int* bl
                     if (rep > 0) ms = std::min(ms, t);   // first launch is the warm-up
                 }
                 if (e != cudaSuccess) break;
-                if (ms < best) { best = ms; bR = refill; bB = blocks; bO = order; }
+                if (ms < kFewer * best || (blocks == bB && ms < best)) { best = ms; bR = refill; bB = blocks; bO = order; }
             }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -386,7 +391,7 @@ extern "C" cudaError_t bhAutotuneBatch(const BHView* views, int n, int* blocksKe
                 cudaEventElapsedTime(&t, e0, e1);
                 if (rep > 0) ms = std::min(ms, t);   // first launch is the warm-up
             }
-            if (e == cudaSuccess && ms < best) { best = ms; bestB = blocks; }
+            if (e == cudaSuccess && ms < kFewer * best) { best = ms; bestB = blocks; }
         }
         bhSetTuning(family, keepR, e == cudaSuccess ? bestB : keepB);
         if (e != cudaSuccess) break;

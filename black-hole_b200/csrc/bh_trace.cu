@@ -26,6 +26,7 @@
 #include "bh_post.cuh"
 #include "bh_internal.h"
 #include "bh_launch.h"
+#include "bh_launch_rules.h"
 
 namespace {
 
@@ -345,7 +346,7 @@ BH_DEV void trace_tile(const TraceParams& P, unsigned tile, unsigned lane, unsig
 
 // One frame (or one pixel list), tile-synchronous: each warp claims 32 ray
 // ids -- one 8x4 tile, or 32 consecutive list entries; fewer where there are few
-// (rays_per_warp) -- at a time (the counter counts tiles) and traces them to the
+// (bh_rays_per_warp) -- at a time (the counter counts tiles) and traces them to the
 // last ray.  This is the FP32
 // render path under the default work distribution (a warp refills only when
 // all 32 lanes are idle); it skips trace_kernel's per-step ballots and result
@@ -566,50 +567,12 @@ ray_set_kernel(const __grid_constant__ RaySet S, int first, int nUnits, unsigned
     }
 }
 
-// Rays a warp of the tile kernel takes at a time.  A small frame lasts as long as the
-// warp of its longest rays, and a warp's steps cost the union of its lanes' paths (disk
-// samples above all, which come at different steps); while the GPU has warps to
-// spare, fewer rays a warp shorten that.  The largest power of two that makes at most
-// 8192 groups (14 a scheduler): 128 x 72 Kerr-Newman 1.19 ms at 32 rays a warp, 1.05 /
-// 1.04 / 1.03 / 0.93 / 0.98 at 16 / 8 / 4 / 2 / 1 (2 taken); 320 x 180 1.92, 1.78 / 1.74 / 1.90 /
-// 2.09 / 3.75 (8 taken); 480 x 270 1.73, 1.64 / 1.76 / 2.32 (16 taken); 640 x 360 1.89, 1.88 /
-// 2.30 (32 taken); Reissner-Nordstroem 128 x 72 0.81 -> 0.47, 320 x 180 0.70 -> 0.59.
-// (A list whose length only the device knows is traced 32 at a time.)
-int rays_per_warp(const TraceParams& P)
-{
-    int width = 32;
-    if (!P.nRaysDev)
-        while (width > 1 && ((unsigned long long)P.nRays * 2u) / (unsigned)width <= 8192u) width >>= 1;
-    return width;
-}
-
-// Warps an SM of the tile kernel for a small or middling frame (0: as many as fit).  Up to some tens
-// of thousands of tiles a frame ends with a few warps whose rays go round the hole; those
-// started first and ran all the while next to 25 .. 28 others, so fewer warps an SM let them
-// through sooner (1283 x 719 Reissner-Nordstroem: the queue empty at 1.17 ms, the last warp,
-// begun at 0, at 1.77).  Geometric means over random views, against all that fit:
-// spherical 96 x 54 to 480 x 270 at 12 warps 1.03 .. 1.08x (8: 1.08 .. 1.14x, but 0.77 .. 0.94x for
-// views that the hole fills), 512 x 288 and 640 x 360 at 12 1.06 .. 1.08x, 960 x 540 at 16 1.03x,
-// 1283 x 719 at 20 1.02x (1.05 .. 1.09x where one ray is the frame), 1920 x 1080 at 24 0.98 ..
-// 1.09x (not taken); rotating up to 160 x 90 at 10 1.07 .. 1.10x (15: 1.04 .. 1.06x), 240 x 135 to
-// 480 x 270 at 15 1.04 .. 1.11x (10: 1.01 .. 1.06x), 512 x 288 .. 960 x 540 at 15 1.03 .. 1.05x,
-// 1283 x 719 at 20 0.99x (not taken).  Fewer still help more at the mean, but cost views without
-// such rays up to 20 %.
-int warps_per_sm(const TraceParams& P, bool kerr)
-{
-    if (P.nRaysDev) return 0;
-    const unsigned tiles = P.nRays / 32u;
-    if (tiles <= 512u && kerr) return 10;
-    if (tiles <= 8192u) return kerr ? 15 : 12;
-    if (tiles <= 16384u) return kerr ? 15 : 16;
-    return tiles <= 32768u && !kerr ? 20 : 0;
-}
-
 template <class Ray, bool STATS>
 cudaError_t launch_one(const TraceParams& P0, int blocksPerSm, cudaStream_t stream)
 {
     TraceParams P = P0;
     P.raysPerWarp = 32;
+    int ruleWarps = 0;
     auto k = trace_kernel<Ray, STATS>;
     constexpr int block = block_of<Ray, STATS>();
     if constexpr (!STATS && sizeof(typename Ray::Real) == 4)
@@ -617,8 +580,8 @@ cudaError_t launch_one(const TraceParams& P0, int blocksPerSm, cudaStream_t stre
         if (P.refillMin >= 32 && !P.dirs)
         {
             k = tile_kernel<Ray>;
-            P.raysPerWarp = rays_per_warp(P);
-            if (blocksPerSm == 0) blocksPerSm = warps_per_sm(P, Ray::kKerrFamily) * 32 / block;
+            P.raysPerWarp = bh_rays_per_warp(P.nRays, !P.nRaysDev);
+            ruleWarps = bh_warps_per_sm(P.nRays, !P.nRaysDev, Ray::kKerrFamily);
         }
     }
     int dev = 0, sms = 0, occ = 0;
@@ -628,8 +591,7 @@ cudaError_t launch_one(const TraceParams& P0, int blocksPerSm, cudaStream_t stre
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, block, 0);
     if (e != cudaSuccess) return e;
-    if (occ < 1) occ = 1;
-    int per = (blocksPerSm > 0 && blocksPerSm < occ) ? blocksPerSm : occ;
+    const int per = bh_blocks_per_sm(occ, ruleWarps, block / 32, blocksPerSm);
     long long need = ((long long)P.nRays * (32 / P.raysPerWarp) + block - 1) / block;
     long long grid = (long long)per * sms;
     if (grid > need) grid = need;

@@ -163,9 +163,10 @@ cudaError_t bhPostProcess(uchar4* out, const float4* accum, float4* bloomA, floa
 
 /* Work-distribution tuning of a metric family (0: Schwarzschild / RN,
  * 1: Kerr / Kerr-Newman): a warp refills its idle lanes once at least
- * `refillMin` (1..32) are idle; `blocksPerSm` CTAs (160 threads for the
- * rotating family, 128 for the spherical one) stay
- * resident per SM (0: as many as occupancy allows).  With refillMin = 32 (the
+ * `refillMin` (1..32) are idle; at most `blocksPerSm` CTAs (160 threads for
+ * the rotating family, 128 for the spherical one) stay resident per SM (0: as
+ * many as occupancy allows).  Single frames of up to 32,768 tiles (rotating:
+ * 16,384) take fewer by a rule of their size, whatever is set.  With refillMin = 32 (the
  * default) FP32 renders run the tile-synchronous kernel (a warp traces one
  * 8x4 tile to its last ray, then takes the next); below 32 they run the
  * refill-queue kernel.  Returns 1 when applied, 0 when a value is out of
@@ -224,7 +225,8 @@ void bhBatchGraphDestroy(BHBatchGraph* graph);
 /* Autotuner: times the FP32 tracing kernel of p's metric family on p's view
  * (blocking, with a temporary HDR buffer) over the resident CTAs per SM, the
  * warp refill threshold and the tile order, applies the fastest setting
- * (bhSetTuning / bhSetTileOrder) and reports it. */
+ * (bhSetTuning / bhSetTileOrder; fewer CTAs than fit only if 1 % faster) and
+ * reports it. */
 cudaError_t bhAutotune(BH_PARAMS_IN p, int* refillMin, int* blocksPerSm, int* tileOrder, float* bestMs);
 
 /* Batch autotuner: for each metric family present in the views, times
