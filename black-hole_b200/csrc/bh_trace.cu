@@ -580,8 +580,10 @@ cudaError_t launch_one(const TraceParams& P0, int blocksPerSm, cudaStream_t stre
         if (P.refillMin >= 32 && !P.dirs)
         {
             k = tile_kernel<Ray>;
-            P.raysPerWarp = bh_rays_per_warp(P.nRays, !P.nRaysDev);
-            ruleWarps = bh_warps_per_sm(P.nRays, !P.nRaysDev, Ray::kKerrFamily);
+            const float dist = sqrtf(P.camPos.x * P.camPos.x + P.camPos.y * P.camPos.y + P.camPos.z * P.camPos.z);
+            const bool wide = bh_wide_view(dist, P.tanHalfFov, P.M, P.diskOn ? P.diskOuter : 0.f);
+            P.raysPerWarp = bh_rays_per_warp(P.nRays, !P.nRaysDev, wide);
+            ruleWarps = bh_warps_per_sm(P.nRays, !P.nRaysDev, Ray::kKerrFamily, wide);
         }
     }
     int dev = 0, sms = 0, occ = 0;
