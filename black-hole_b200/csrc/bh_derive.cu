@@ -23,8 +23,9 @@
 //     is evaluated first, and then all radii between those within kWindow of the
 //     lowest.  Near the minimum the energies of neighbouring visits differ by less
 //     than their rounding, so the window is evaluated exactly as the scan does it.
-//     A naked singularity, or a hole without a valid coarse radius, gets the whole
-//     scan.
+//     A naked singularity, a hole without a valid coarse radius, and masses outside
+//     kMassLow .. kMassHigh get the whole scan: far outside, products of an energy
+//     leave FP32's normal range, and below 1e-6 the scan starts inside the horizon.
 // Bound: instruction issue (the IEEE divisions and roots of ~2,600 energies a hole)
 // with one thread's set-up before it.  13,824 holes: 4.39 ms with the running sum
 // (a chain of 12,000 dependent sums a hole) and the whole scan, 0.19 ms so.
@@ -38,6 +39,7 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kStride = 16;           // coarse pass of the scan
 constexpr float kWindow = 1e-3f;      // relative: coarse radii this close to the lowest energy mark the window
+constexpr float kMassLow = 1e-5f, kMassHigh = 1e5f;
 constexpr int kMaxSegments = 64;
 constexpr float kExtremal = 0.995f;
 constexpr float kNakedCap = 2.25f;
@@ -121,12 +123,12 @@ struct Segment
 };
 
 // The visiting sequence of `for (r = rStart; r <= rEnd; r += dr)` as exact
-// arithmetic sequences; returns the number of segments, the visits in *total.
+// arithmetic sequences, as far as r is finite; returns the number of segments, the visits in *total.
 __device__ int scan_segments(float rStart, float rEnd, float dr, Segment* seg, int* total)
 {
     int m = 0, k = 0;
     float r = rStart;
-    while (r <= rEnd && m < kMaxSegments)
+    while (r <= rEnd && r <= 3.402823466e38f && m < kMaxSegments)
     {
         // ulp of r's binade and its upper end, in ulps 2^24 (normal numbers)
         const int e = max((__float_as_int(r) >> 23) & 255, 1);
@@ -138,7 +140,7 @@ __device__ int scan_segments(float rStart, float rEnd, float dr, Segment* seg, i
         seg[m++] = Segment{r, 0.f, k, 1};
         ++k;
         r = r1;
-        if (!same || !(r1 <= rEnd) || m >= kMaxSegments) continue;
+        if (!same || !(r1 <= rEnd) || m >= kMaxSegments) continue;    // (r1 infinite: another exponent)
         const int i1 = (int)((double)r1 * perUlp), inc = (int)fmin((double)step * perUlp, (double)top);
         if (inc < 1) break;
         const int lim = (int)fmin((double)rEnd * perUlp, (double)(top - 1));   // last multiple a visit may take
@@ -180,6 +182,7 @@ derive_kernel(BHDeriveRequest* __restrict__ req, BHDerived* __restrict__ out, in
     __shared__ Segment seg[kMaxSegments];
     __shared__ float sE[kThreads / 32], sLow;
     __shared__ int sK[kThreads / 32], sTotal, sLo, sHi;
+    __shared__ bool sWindow;
     __shared__ BHDerived sD;
     __shared__ float sM, sRp, sA, sQ;
     const int i = blockIdx.x;
@@ -213,13 +216,15 @@ derive_kernel(BHDeriveRequest* __restrict__ req, BHDerived* __restrict__ out, in
         }
         d.a = fm(aEff, M);
         d.Q = fm(qEff, M);
-        d.naked = fs(fs(fm(M, M), fm(d.a, d.a)), fm(d.Q, d.Q)) < 0.f ? 1 : 0;
+        const float disc = fs(fs(fm(M, M), fm(d.a, d.a)), fm(d.Q, d.Q));   // NaN for a spinning M above 1.8e19
+        d.naked = disc < 0.f ? 1 : 0;
         d.rPlus = d.naked ? 0.f : outerHorizon(M, d.a, d.Q);
         if (threadIdx.x == 0)
         {   // iscoRadius
-            const float rp = d.naked ? fm(kSingCut, M) : d.rPlus;
+            const float rp = disc >= 0.f ? d.rPlus : fm(kSingCut, M);
             sRp = rp;
             sM = M;
+            sWindow = disc >= 0.f && M >= kMassLow && M <= kMassHigh;
             sLo = 0x7fffffff;
             sHi = -1;
             scan_segments(rp > 1e-6f ? fm(rp, 1.02f) : fm(0.5f, M), fm(12.f, M), fm(0.001f, M), seg, &sTotal);
@@ -250,7 +255,7 @@ derive_kernel(BHDeriveRequest* __restrict__ req, BHDerived* __restrict__ out, in
     float bestE = 1e30f;
     int bestK = 0x7fffffff;
     int lo = 0, hi = total;               // visits to evaluate
-    if (!sD.naked)
+    if (sWindow)
     {
         int at = 0;
         for (int k = (int)threadIdx.x * kStride; k < total; k += kThreads * kStride)
