@@ -140,6 +140,7 @@ struct BHSurrogate
     unsigned char* setDev[2] = {nullptr, nullptr};
     unsigned short* setOrder[2] = {nullptr, nullptr};
     cudaEvent_t setDone[2] = {nullptr, nullptr};
+    cudaEvent_t setFork = nullptr, setJoin = nullptr;   // not the frames': a frame may be queued by another thread
     size_t setUnits = 0;
     bool setPinned = false;
     // anchored frames: RK4 anchors every anchorStride pixels (0: the network's own directions)
@@ -185,6 +186,8 @@ cudaError_t ensureRaySets(BHSurrogate* s, size_t units, int sets)
     freeRaySets(s);
     cudaError_t e = cudaSuccess;
     if (!s->aux) e = cudaStreamCreateWithFlags(&s->aux, cudaStreamNonBlocking);
+    if (e == cudaSuccess && !s->setFork) e = cudaEventCreateWithFlags(&s->setFork, cudaEventDisableTiming);
+    if (e == cudaSuccess && !s->setJoin) e = cudaEventCreateWithFlags(&s->setJoin, cudaEventDisableTiming);
     for (int k = 0; k < sets && e == cudaSuccess; ++k)
     {
         s->setPinned = sets > 1;
@@ -212,6 +215,8 @@ void freeAll(BHSurrogate* s)
     freeRaySets(s);
     if (s->evFork) cudaEventDestroy(s->evFork);
     if (s->evJoin) cudaEventDestroy(s->evJoin);
+    if (s->setFork) cudaEventDestroy(s->setFork);
+    if (s->setJoin) cudaEventDestroy(s->setJoin);
     if (s->aux) cudaStreamDestroy(s->aux);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -725,14 +730,14 @@ cudaError_t bhSurrogateGenerate(BHSurrogate* s, long long rays, int views, unsig
                             (size_t)(v1 - v0 + 1) * sizeof(RayView) + k * sizeof(RayUnit), cudaMemcpyHostToDevice,
                             s->stream);
         if (e == cudaSuccess) e = bh_sort_ray_set(set, s->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(s->evFork, s->stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(s->aux, s->evFork, 0);
+        if (e == cudaSuccess) e = cudaEventRecord(s->setFork, s->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s->aux, s->setFork, 0);
         if (e == cudaSuccess) e = bh_device_counter(&cKerr);
         if (e == cudaSuccess) e = bh_device_counter(&cSph);
         if (e == cudaSuccess) e = bh_trace_ray_set(set, true, cKerr, s->stream);
         if (e == cudaSuccess) e = bh_trace_ray_set(set, false, cSph, s->aux);
-        if (e == cudaSuccess) e = cudaEventRecord(s->evJoin, s->aux);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(s->stream, s->evJoin, 0);
+        if (e == cudaSuccess) e = cudaEventRecord(s->setJoin, s->aux);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s->stream, s->setJoin, 0);
         if (e == cudaSuccess) e = cudaEventRecord(s->setDone[turn], s->stream);
     }
     const cudaError_t e2 = cudaStreamSynchronize(s->stream);
