@@ -680,6 +680,7 @@ cudaError_t bhSurrogateGenerate(BHSurrogate* s, long long rays, int views, unsig
     if (dReq) cudaFree(dReq);
     if (dHoles) cudaFree(dHoles);
 
+    if (e == cudaSuccess) S.dsN = 0;      // rows are overwritten from here: no set until all are
     int turn = 0;
     for (size_t u0 = 0; u0 < units && e == cudaSuccess; u0 += chunk, turn ^= 1)
     {
@@ -741,7 +742,9 @@ cudaError_t bhSurrogateGenerate(BHSurrogate* s, long long rays, int views, unsig
         if (e == cudaSuccess) e = cudaEventRecord(s->setDone[turn], s->stream);
     }
     const cudaError_t e2 = cudaStreamSynchronize(s->stream);
-    if (e == cudaSuccess) e = e2;
+    // after an error the main stream may not have waited for the other one, which writes the rows too
+    const cudaError_t e3 = s->aux ? cudaStreamSynchronize(s->aux) : cudaSuccess;
+    if (e == cudaSuccess) e = e2 == cudaSuccess ? e3 : e2;
     if (e == cudaSuccess) S.dsN = rays;
     return e;
 }
