@@ -12,6 +12,7 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <random>
 #include <vector>
 #include <cuda_runtime.h>
@@ -627,7 +628,7 @@ cudaError_t bhSurrogateGradients(BHSurrogate* s, const float* in, const float* t
     return e;
 }
 
-cudaError_t bhSurrogateGenerate(BHSurrogate* s, long long rays, int views, unsigned seed)
+static cudaError_t generateRaySet(BHSurrogate* s, long long rays, int views, unsigned seed)
 {
     if (!s || rays <= 0 || views <= 0 || rays % views) return cudaErrorInvalidValue;
     SgState& S = s->S;
@@ -747,6 +748,13 @@ cudaError_t bhSurrogateGenerate(BHSurrogate* s, long long rays, int views, unsig
     if (e == cudaSuccess) e = e2 == cudaSuccess ? e3 : e2;
     if (e == cudaSuccess) S.dsN = rays;
     return e;
+}
+
+// the views' parameters are host vectors, whose allocation may throw
+cudaError_t bhSurrogateGenerate(BHSurrogate* s, long long rays, int views, unsigned seed)
+{
+    try { return generateRaySet(s, rays, views, seed); }
+    catch (const std::bad_alloc&) { return cudaErrorMemoryAllocation; }
 }
 
 cudaError_t bhSurrogateDataset(BHSurrogate* s, const float** in, const float** tgt, long long* n)
