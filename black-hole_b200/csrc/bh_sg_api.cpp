@@ -134,6 +134,8 @@ struct BHSurrogate
     bool critValid = false;
     CritKey critKey;
     float crit[kCritBins];
+    float* fwdIn = nullptr;           // copy of a forward pass's inputs that its outputs overwrite
+    int fwdCap = 0;
     // ray sets: views and units of one launch (two sets in turn: the host fills one while the GPU
     // traces the other), their rays' tracing order
     cudaStream_t aux = nullptr;       // the spherical family beside the Kerr family
@@ -210,7 +212,7 @@ void freeAll(BHSurrogate* s)
     sg_free_batch(S);
     void* ps[] = {S.params, S.grads, S.adamM, S.adamV, S.W, S.Wt, S.biasPacked, S.loss, S.dsIn, S.dsTgt, s->list,
                   s->counters, s->heldPix, s->heldPred, s->anchorPix, s->anchorRecIdx, s->anchorRec,
-                  s->cellPix, s->cellGate, s->sampleDir, s->samplePix, s->blockOrder};
+                  s->fwdIn, s->cellPix, s->cellGate, s->sampleDir, s->samplePix, s->blockOrder};
     for (void* p : ps)
         if (p) cudaFree(p);
     freeRaySets(s);
@@ -602,6 +604,24 @@ cudaError_t bhSurrogateForward(BHSurrogate* s, const float* in, float* out, int 
     {
         SgInferArgs a{S.W, S.W + 4 * kHidW, S.biasPacked, in, out, (unsigned)n, S.err};
         return sg_infer_launch(a, nullptr, stream);
+    }
+    // a CTA's outputs may lie where another still reads its inputs: then from a copy of them
+    const char *i0 = reinterpret_cast<const char*>(in), *o0 = reinterpret_cast<const char*>(out);
+    if (i0 < o0 + (size_t)n * 16 * sizeof(float) && o0 < i0 + (size_t)n * 8 * sizeof(float))
+    {
+        cudaError_t e = cudaSuccess;
+        if (n > s->fwdCap)
+        {
+            if (s->fwdIn) cudaFree(s->fwdIn);
+            s->fwdIn = nullptr;
+            s->fwdCap = 0;
+            e = bh_device_alloc(reinterpret_cast<void**>(&s->fwdIn), (size_t)n * 8 * sizeof(float));
+            if (e != cudaSuccess) return e;
+            s->fwdCap = n;
+        }
+        e = cudaMemcpyAsync(s->fwdIn, in, (size_t)n * 8 * sizeof(float), cudaMemcpyDeviceToDevice, stream);
+        if (e != cudaSuccess) return e;
+        in = s->fwdIn;
     }
     return sg_chain_forward(S, in, out, n, stream);
 }
