@@ -26,8 +26,8 @@
 // all five products: a CTA takes one 128-row tile of one product over one part of the
 // batch, an accumulator per share of it.  An accumulator's error grows with its rows (against FP64 over the
 // same BF16 operands 5.0e-7 to 5.6e-7 with shares of 512, 1.1e-6 to 1.3e-6 with 14 of 1,170).  16,384 rows:
-// 24 us (20.7 us with those 14, added by reductions in an order that changed from run to run; 26.6 + 4 x 31 us
-// a product at a time, and ten transposes of 12.4).
+// 21.3 us (24.4 us with the shares added to the part in L2; 20.7 us with those 14, added by reductions in an
+// order that changed from run to run; 26.6 + 4 x 31 us a product at a time, and ten transposes of 12.4).
 // ---------------------------------------------------------------------------
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -403,7 +403,7 @@ chain_kernel(const __grid_constant__ ChainMaps M, const __grid_constant__ ChainA
 }
 
 // ---- weight gradients ----------------------------------------------------------
-constexpr int kGradStages = 4, kGradThreads = 192;        // four epilogue warps, TMA, MMA
+constexpr int kGradStages = 4, kGradThreads = 576;        // sixteen epilogue warps, TMA, MMA
 constexpr uint32_t kBox = 64u * 128u;                     // 64 batch rows x 64 columns
 constexpr uint32_t kGradStage = 6u * kBox;                // 2 boxes of one operand, up to 4 of the other
 constexpr uint32_t kGradSmem = kGradStages * kGradStage + 1024u;
@@ -417,11 +417,6 @@ __device__ __forceinline__ uint64_t sdesc_mn_sw128(uint32_t saddr)
            ((uint64_t)1u << 46) | ((uint64_t)2u << 61);
 }
 
-__device__ __forceinline__ void red4(float* p, float a, float b, float c, float d)
-{
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
 struct GradMaps
 {
     CUtensorMap rows[kLayers];   // the operand whose columns are the tile's rows: dZ_l; X of the head
@@ -433,7 +428,8 @@ __device__ __forceinline__ int share_tile(int tiles, int shares, int k) { return
 
 // Tile t = 2 l + h: rows 128 h .. of product l.  The head's is X^T dY (its gradient's transpose).
 // blockIdx.y: the part.  Its shares' products go to the two accumulators in turn, so one share is
-// read back and added while the next is multiplied.  The first warps also add the slices of the biases.
+// read back and added in registers while the next is multiplied.  The first warps also add the slices
+// of the biases.
 __global__ void __launch_bounds__(kGradThreads, 1)
 weight_grad_kernel(const __grid_constant__ GradMaps maps, const float* slices, float* parts, int tiles,
                    unsigned* __restrict__ err)
@@ -455,7 +451,7 @@ weight_grad_kernel(const __grid_constant__ GradMaps maps, const float* slices, f
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < kGradStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&done[b], 1); mbar_init(&taken[b], 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&done[b], 1); mbar_init(&taken[b], 16); }
         fence_barrier_init();
         tma_prefetch_desc(tA);
         tma_prefetch_desc(tB);
@@ -469,7 +465,7 @@ weight_grad_kernel(const __grid_constant__ GradMaps maps, const float* slices, f
     wait_for_previous();
     const uint32_t tmem = tmemSlot;
 
-    if (threadIdx.x == 128)
+    if (threadIdx.x == 512)
     {
         const int first = 2 * share_tile(tiles, shares, k0), blocks = 2 * share_tile(tiles, shares, k1) - first;
         int issued = 0;
@@ -488,7 +484,7 @@ weight_grad_kernel(const __grid_constant__ GradMaps maps, const float* slices, f
         for (int kb = issued > kGradStages ? issued - kGradStages : 0; kb < issued; ++kb)
             if (!mbar_wait(&full[kb % kGradStages], (kb / kGradStages) & 1, err)) break;
     }
-    else if (threadIdx.x == 160)
+    else if (threadIdx.x == 544)
     {
         const uint32_t idesc = idesc_bf16_f32(head ? 64 : 256) | (1u << 15) | (1u << 16);   // A and B MN-major
         bool ok = true;
@@ -514,10 +510,10 @@ weight_grad_kernel(const __grid_constant__ GradMaps maps, const float* slices, f
             mma_commit(&done[buf]);
         }
     }
-    else if (warp < 4)
+    else if (warp < 16)
     {
         // this tile's biases, one a thread (the head's first tile: its 16 and the loss's 8)
-        if (!head || (m0 == 0 && threadIdx.x < kOut + 8))
+        if (threadIdx.x < (head ? (m0 == 0 ? kOut + 8 : 0) : 128))
         {
             const float* from = slices + (head ? kHidden * kWidth : l * kWidth + m0) + threadIdx.x;
             float sum = 0.f;
@@ -531,32 +527,33 @@ weight_grad_kernel(const __grid_constant__ GradMaps maps, const float* slices, f
             part[SgLayout::b(l) + m0 + threadIdx.x] = sum;
         }
         __syncwarp();
-        // four columns of a row are a float4, the rows of a tile follow one another (sg_quad).  A float4 is
-        // one thread's: stored with the first share, then added to in the shares' order
-        const uint32_t tl = tmem + ((uint32_t)(warp * 32) << 16);
-        float* g = part + SgLayout::w(l) + m0 * (head ? kOut : kWidth) + 4 * (warp * 32 + lane);
-        for (int k = k0; k < k1; ++k)
+        // a row and 64 columns a thread (the head: 16, of the first four warps)
+        const int c0 = (warp >> 2) * 64, cols = !head ? 64 : c0 == 0 ? kOut : 0, row = (warp & 3) * 32 + lane;
+        const uint32_t tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
+        float acc[64] = {};
+        bool ok = true;
+        for (int k = k0; k < k1 && ok; ++k)
         {
             const int turn = k - k0, buf = turn & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(&done[buf], (uint32_t)(turn >> 1) & 1u, err))) break;
+            ok = __all_sync(0xffffffffu, mbar_wait(&done[buf], (uint32_t)(turn >> 1) & 1u, err));
             tc_fence_after();
-#pragma unroll 1
-            for (int c = 0; c < (head ? kOut : kWidth); c += 16)
-            {
-                __syncwarp();
-                float v[16];
-                tmem_ld16(tl + (uint32_t)(buf * 256 + c), v);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+            for (int c = 0; c < 64; c += 16)
+                if (c < cols && ok)
                 {
-                    float* at = g + (c / 4 + i) * 512;
-                    if (turn == 0) *reinterpret_cast<float4*>(at) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                    else red4(at, v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    float v[16];
+                    tmem_ld16(tl + (uint32_t)(buf * 256 + c), v);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) acc[c + i] += v[i];
                 }
-            }
             tc_fence_before();
             if (lane == 0) mbar_arrive(&taken[buf]);
         }
+        // four columns of a row are a float4, the rows of a tile follow one another (sg_quad)
+        float4* g = reinterpret_cast<float4*>(part + SgLayout::w(l)) + (m0 / 4) * (head ? kOut : kWidth) + c0 * 32 + row;
+#pragma unroll
+        for (int c = 0; c < 64; c += 4)
+            if (c < cols && ok) g[c * 32] = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
     }
     __syncwarp();
     tc_fence_before();

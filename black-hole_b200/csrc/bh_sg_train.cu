@@ -12,7 +12,7 @@
 // dX_l reads W_l^T, kept next to W_l after every update.  A step is three launches: the
 // passes of 128 rays a CTA and the parts of all gradients (bh_sg_chain.cu), and Adam, which adds
 // the parts, with the packing of the BF16 weights; each starts while the one before it ends
-// (set-up, and the features of the next batch).  16,384 rays: 107 us (97 us with sums in an order that changed from
+// (set-up, and the features of the next batch).  16,384 rays: 103 us (97 us with sums in an order that changed from
 // run to run; 710 us as 36 launches).
 // No counterpart in the reference (it has no learned component).
 // ---------------------------------------------------------------------------
