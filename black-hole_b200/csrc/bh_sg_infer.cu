@@ -31,7 +31,7 @@
 // warp and turn) and 1000 for the cluster-scope arrival; features 5300 a tile.  All
 // column indexes of the epilogue and the features are constants, accumulators load while
 // the columns before are turned, and a wait reads the timer only after it ran out once:
-// 2,000,003 rays 1.292 -> 1.218 ms (the features' inputs were indexed through local memory).
+// 2,000,003 rays a call 1.355 -> 1.285 ms (the features' inputs were indexed through local memory).
 // ---------------------------------------------------------------------------
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -3,8 +3,9 @@
 // tensor memory (TMEM) allocation, UMMA shared-memory and instruction
 // descriptors, tcgen05.mma / commit / ld, TMA tiled loads and mbarriers.
 //
-// Conventions used by every kernel here:
-//  * operands are BF16, K-major (the contraction index is contiguous), staged
+// Conventions used by the kernels here:
+//  * operands are BF16, K-major (the contraction index is contiguous; only
+//    weight_grad_kernel reads MN-major ones, with descriptors of its own), staged
 //    in shared memory in the 128-byte-swizzle layout: a tile of R rows x 64
 //    columns is R rows of 128 B, grouped in 8-row / 1024-B atoms, the 16-B
 //    chunk index inside a row XOR-ed with (row % 8).  TMA with
