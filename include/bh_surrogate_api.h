@@ -88,7 +88,8 @@ cudaError_t bhSurrogateFeatures(const float* in, void* features, int n, cudaStre
 
 /* Head outputs (n x 16 floats) of n input rows.  fused != 0: the fused
  * persistent tensor-core kernel used for rendering; fused == 0: the training
- * form (the kernel of the training passes, without their stores). */
+ * form (the kernel of the training passes, without their stores); `out` may
+ * then overlap `in` (the inputs are copied first). */
 cudaError_t bhSurrogateForward(BHSurrogate* s, const float* in, float* out, int n, int fused, cudaStream_t stream);
 
 /* Forward, loss and backward on n rays (n a multiple of 128; device inputs
@@ -110,7 +111,7 @@ cudaError_t bhSurrogateGradients(BHSurrogate* s, const float* in, const float* t
  * inclination U(2, 88) deg; azimuth U(0, 360) deg; vertical FOV U(30, 90)
  * deg, 16:9; disk on; balanced preset), directions uniform over each view's
  * screen, all from `seed`; the ray set (inputs and targets) stays in device
- * memory (blocking). */
+ * memory (blocking).  After an error the set is the one before, or none. */
 cudaError_t bhSurrogateGenerate(BHSurrogate* s, long long rays, int views, unsigned seed);
 
 /* Device pointers to the current ray set (rows of 8 floats) and its size. */
@@ -123,7 +124,8 @@ cudaError_t bhSurrogateDatasetCopy(BHSurrogate* s, float* in, float* tgt, long l
 /* `steps` Adam steps (beta 0.9 / 0.999) on batches of `batch` rays (a
  * multiple of 128) drawn from the ray set by a hash of (seed, step); the
  * learning rate decays from lr to lr / 20 on a cosine.  lossHistory (may be
- * null) receives 5 batch-mean loss terms per step (blocking). */
+ * null) receives 5 batch-mean loss terms per step (blocking).  All sums are
+ * added in an order fixed by the batch, so the same calls repeat bit for bit. */
 cudaError_t bhSurrogateTrain(BHSurrogate* s, int steps, int batch, float lr, unsigned seed, float* lossHistory);
 
 /* Render one frame with the surrogate: same buffers and result layout as
